@@ -28,19 +28,68 @@ __host__ __device__ constexpr inline int smem_ld(int N) { return (N % 2 == 0) ? 
 // fragment loads of the flush are free of bank conflicts
 __host__ __device__ constexpr inline int panel_ld(int N) { return N + ((4 - N % 16) + 16) % 16; }
 
-// leading dimension of the resident G of k_interval: = 2 (mod 8) doubles, so that the DMMA
-// accumulator tiles of the rank updates (lane 4g+q at row g, columns 2q, 2q+1) are free of
-// bank conflicts
-__host__ __device__ constexpr inline int interval_ld(int N) { return N + ((2 - N % 8) + 8) % 8; }
+// N rounded up to whole DMMA tiles of 16 rows; the 8-column tiles of N columns, one more where
+// their count is a multiple of neither 2 nor 3 (the flush takes strips of 2 or 3 tiles)
+__host__ __device__ constexpr inline int pad16(int N) { return (N + 15) & ~15; }
+__host__ __device__ constexpr inline int tile_cols(int N) {
+  const int t = (N + 7) / 8;
+  return t % 2 != 0 && t % 3 != 0 ? t + 1 : t;
+}
 
-// bytes of dynamic shared memory of k_interval for a chain of size N with delay depth kmax
-// (matrix in smem when `resident`)
+// leading dimension of a G resident in shared memory: whole 16-row tiles and = 2 (mod 16) doubles,
+// so that the DMMA accumulator tiles of the rank updates (lane 4g+q at row g, columns 2q, 2q+1) and
+// the 16-byte accesses of lanes that walk columns are free of bank conflicts
+__host__ __device__ constexpr inline int interval_ld(int N) { return pad16(N) + 2; }
+// doubles of a resident G: columns padded to the tiles of the flush
+__host__ __device__ constexpr inline size_t resident_doubles(int N) { return (size_t)interval_ld(N) * 8 * tile_cols(N); }
+
+// doubles of the interval body's work area (the panels X and Y, or the stage of the dense
+// exp(-dt K)): an even number, so that what follows stays 16-byte aligned
+__host__ __device__ constexpr inline size_t interval_work_doubles(int N, int kmax) {
+  const size_t panels = (size_t)panel_ld(pad16(N)) * kmax * 2;
+  const size_t stage = (size_t)8 * (pad16(N) + 4);
+  return panels > stage ? panels : stage;
+}
+
+// Dynamic shared memory of the interval body, in doubles, for a chain of N sites whose panels hold
+// kmax flips (a resident chain's always 16, so that the layout depends on N alone)
+struct IntervalLayout {
+  size_t G, work, Y, rec, dl, thr, u, rr, vp, vm, fields, pw, ints, total;
+};
+constexpr int kRecordDoubles = 2 * 16 * 18 + 2 * 16;  // the walk's records, gammas and the words idle lanes write to
+__host__ __device__ constexpr inline IntervalLayout interval_layout(int N, int kmax, bool resident) {
+  IntervalLayout o{};
+  if (resident) kmax = 16;
+  size_t p = 0;
+  o.G = p; p += resident ? resident_doubles(N) : 0;
+  o.work = p; p += interval_work_doubles(N, kmax);             // X, then Y; or the stage
+  o.Y = o.work + (size_t)panel_ld(pad16(N)) * kmax;
+  o.rec = p; p += kRecordDoubles;                              // the walk's records (16-byte aligned)
+  o.ints = p; p += 10;                                         // accepted counts (4), accepted sites (16)
+  o.dl = p; p += N;
+  o.thr = p; p += N;
+  o.u = p; p += N;
+  o.rr = p; p += N;
+  o.vp = p; p += N;
+  o.vm = p; p += N;
+  o.fields = p; p += (size_t)(2 * N + 7) / 8;                  // int8 fields and flip flags
+  o.pw = p; p += (size_t)(N + 1) / 2;                          // uint32 jump-ahead powers
+  o.total = (p + 1) & ~size_t(1);
+  return o;
+}
 __host__ __device__ inline size_t interval_smem_doubles(int N, int kmax, bool resident) {
-  const size_t mat = resident ? (size_t)N * interval_ld(N) : 0;
-  const size_t panels = (size_t)panel_ld(N) * kmax * 2;
-  const size_t stage = (size_t)8 * (((N + 15) & ~15) + 4);
-  const size_t work = panels > stage ? panels : stage;
-  return mat + work + 3 * (size_t)N + (size_t)(N + 7) / 4 + (size_t)(N + 1) / 2 + 64;
+  return interval_layout(N, kmax, resident).total;
+}
+
+// A pointer into the block's dynamic shared memory rebased on the shared symbol, so that the
+// accesses through it are shared-memory instructions also inside functions that receive it as a
+// generic pointer (generic accesses took the walk of a site block from 3.0k to 6.0k cycles and
+// the panels from 1k to 3k).
+template <class T>
+__device__ __forceinline__ T* as_shared(T* p) {
+  extern __shared__ __align__(16) double smem[];
+  return reinterpret_cast<T*>(reinterpret_cast<char*>(smem) +
+                              (reinterpret_cast<const char*>(p) - reinterpret_cast<const char*>(smem)));
 }
 
 // ---------------------------------------------------------------------------------
@@ -225,51 +274,98 @@ static __device__ void flush_panels(double* G, int ld, int N, const double* X, i
   rank_update(G, ld, N, N, X, ldx, Y, ldy, k);
 }
 
+}  // namespace hq
+#include "hq_sep.cuh"
+namespace hq {
+
+// vp[i] = e^{V_i}, vm[i] = e^{-V_i} of the fields s[0:N) (each where non-null). Every thread calls
+// it; a barrier must precede their use.
+__device__ __forceinline__ void slice_factors(const HqChain& ch, const int8_t* s, double* vp, double* vm) {
+  for (int i = threadIdx.x; i < ch.N; i += blockDim.x) {
+    const bool pos = s[i] > 0;
+    if (vp) vp[i] = pos ? ch.ev_p : ch.ev_m;
+    if (vm) vm[i] = pos ? ch.ev_m : ch.ev_p;
+  }
+}
+
+// M <- diag(v) M / M <- M diag(v)
+__device__ __forceinline__ void scale_rows(double* M, int ld, int N, const double* v) {
+  HQ_FOR_EACH_ELEM(N, i, j) M[i + (size_t)j * ld] *= v[i];
+}
+__device__ __forceinline__ void scale_cols(double* M, int ld, int N, const double* v) {
+  HQ_FOR_EACH_ELEM(N, i, j) M[i + (size_t)j * ld] *= v[j];
+}
+
+// M <- e^{V} expK M (AFTER true) or expK e^{V} M (AFTER false), v = e^{V}, by the dense or the
+// separable form. RES: M in shared memory with the leading dimension ldr(N) (a compile-time value
+// per lattice size); otherwise any leading dimension. Ends with a barrier.
+enum SideOp { LEFT_B, LEFT_BT, RIGHT_BINV };  // e^V E M,  E e^V M,  M E^-1 e^-V
+template <int OP, bool RES, int PAD>
+__device__ __forceinline__ void apply_side(const HqChain& ch, double* M, int ld, const double* v, double* stage) {
+  if (ch.expk_mode == HQK_EXPK_SEPARABLE) {
+    for_lattice(ch.L, [&](auto lc) {
+      constexpr int L = decltype(lc)::value, N = L * L;
+      constexpr int LD = !RES || L > 12 ? 0 : (PAD ? interval_ld(N) : smem_ld(N));
+      if constexpr (OP == LEFT_B) sep_one<L, LD, 0, 2>(M, ld, ch.sep_a, ch.sep_c, v);
+      else if constexpr (OP == LEFT_BT) sep_one<L, LD, 0, 1>(M, ld, ch.sep_a, ch.sep_c, v);
+      else sep_one<L, LD, 1, 2>(M, ld, ch.sep_ai, ch.sep_ci, v);
+    });
+  } else if constexpr (OP == LEFT_B) {
+    dense_apply(M, ld, ch.N, ch.expK, stage);
+    scale_rows(M, ld, ch.N, v);
+    __syncthreads();
+  } else if constexpr (OP == LEFT_BT) {
+    scale_rows(M, ld, ch.N, v);
+    __syncthreads();
+    dense_apply(M, ld, ch.N, ch.expK, stage);
+  } else {
+    dense_apply_right(M, ld, ch.N, ch.inv_expK, stage);
+    scale_cols(M, ld, ch.N, v);
+    __syncthreads();
+  }
+}
+
 // ---------------------------------------------------------------------------------
 //  wrap of G by B(l) (src/dqmc_core.cpp:142-161, src/hubbard.cpp:293-331)
 //   up  : G <- e^{V_l} E G E^{-1} e^{-V_l}
 //   down: G <- E^{-1} e^{-V_l} G e^{V_l} E
+//  vp = e^{V_l}, vm = e^{-V_l}. With acc_meas (separable mode only) the equal-time estimators ride
+//  on the wrap: up, on the first pass's loads (the G before this wrap); down, on the last pass's
+//  stores (the G after it). RES: G in shared memory with leading dimension interval_ld(N).
 // ---------------------------------------------------------------------------------
-// With acc_meas (separable mode only) the equal-time estimators ride on the wrap: up, on the
-// first pass's loads (the G before this wrap); down, on the last pass's stores (the G after it).
-__device__ __forceinline__ void wrap_slice(const HqChain& ch, double* G, int ld, const int8_t* s, int dir, double* stage,
-                                           double* acc_meas = nullptr, double* red = nullptr) {
+// whether the wrap of lattice size L can measure: small lattices keep G out of shared memory only
+// beside larger chains of the same context, where a pass of its own is as good
+template <bool RES>
+__host__ __device__ constexpr bool wrap_measures(int L) { return RES || L > 12; }
+template <bool RES>
+__device__ __forceinline__ void wrap_slice(const HqChain& ch, double* G, int ld, const double* vp, const double* vm, int dir,
+                                           double* stage, double* acc_meas = nullptr, double* red = nullptr) {
   const int N = ch.N;
   if (ch.expk_mode == HQK_EXPK_SEPARABLE) {
-    // the e^{+-V} scalings ride on the last pass (up) or on the first pass (down)
-    if (dir == HQ_UP) {
-      if (acc_meas)
-        sep_apply_any<0, 0, 1, 0>(G, ld, N, ch.L, ch.sep_a, ch.sep_c, 0, nullptr, 1.0, 1.0, 1.0, 1.0, acc_meas, red);
-      else
-        sep_apply_any(G, ld, N, ch.L, ch.sep_a, ch.sep_c, 0);
-      sep_apply_any<0, 2>(G, ld, N, ch.L, ch.sep_ai, ch.sep_ci, 1, s, ch.ev_p, ch.ev_m, ch.ev_m, ch.ev_p);
-    } else {
-      sep_apply_any<1, 0>(G, ld, N, ch.L, ch.sep_ai, ch.sep_ci, 0, s, ch.ev_m, ch.ev_p, ch.ev_p, ch.ev_m);
-      if (acc_meas)
-        sep_apply_any<0, 0, 0, 2>(G, ld, N, ch.L, ch.sep_a, ch.sep_c, 1, nullptr, 1.0, 1.0, 1.0, 1.0, acc_meas, red);
-      else
-        sep_apply_any(G, ld, N, ch.L, ch.sep_a, ch.sep_c, 1);
-    }
+    for_lattice(ch.L, [&](auto lc) {
+      constexpr int L = decltype(lc)::value;
+      constexpr int LD = !RES || L > 12 ? 0 : interval_ld(L * L);
+      constexpr int kMeas = wrap_measures<RES>(L) ? 1 : 0;
+      if (dir == HQ_UP) {
+        if (kMeas && acc_meas) sep_wrap<L, LD, 1, kMeas>(G, ld, ch, vp, vm, acc_meas, red);
+        else sep_wrap<L, LD, 1, 0>(G, ld, ch, vp, vm, nullptr, red);
+      } else {
+        if (kMeas && acc_meas) sep_wrap<L, LD, 0, kMeas>(G, ld, ch, vp, vm, acc_meas, red);
+        else sep_wrap<L, LD, 0, 0>(G, ld, ch, vp, vm, nullptr, red);
+      }
+    });
     return;
   }
   if (dir == HQ_UP) {
-    apply_expk(ch, G, ld, 0, false, stage);
-    apply_expk(ch, G, ld, 1, true, stage);
-    HQ_FOR_EACH_ELEM(N, i, j) {
-      const double fi = s[i] > 0 ? ch.ev_p : ch.ev_m;
-      const double fj = s[j] > 0 ? ch.ev_m : ch.ev_p;
-      G[i + (size_t)j * ld] *= fi * fj;
-    }
+    dense_apply(G, ld, N, ch.expK, stage);
+    dense_apply_right(G, ld, N, ch.inv_expK, stage);
+    HQ_FOR_EACH_ELEM(N, i, j) G[i + (size_t)j * ld] *= vp[i] * vm[j];
     __syncthreads();
   } else {
-    HQ_FOR_EACH_ELEM(N, i, j) {
-      const double fi = s[i] > 0 ? ch.ev_m : ch.ev_p;
-      const double fj = s[j] > 0 ? ch.ev_p : ch.ev_m;
-      G[i + (size_t)j * ld] *= fi * fj;
-    }
+    HQ_FOR_EACH_ELEM(N, i, j) G[i + (size_t)j * ld] *= vm[i] * vp[j];
     __syncthreads();
-    apply_expk(ch, G, ld, 0, true, stage);
-    apply_expk(ch, G, ld, 1, false, stage);
+    dense_apply(G, ld, N, ch.inv_expK, stage);
+    dense_apply_right(G, ld, N, ch.expK, stage);
   }
 }
 

@@ -3,7 +3,7 @@
 //     std::bernoulli_distribution / generate_canonical<double,53> of libstdc++),
 //     replayed exactly with jump-ahead so every site of a slice gets its uniform at once;
 //   * FP64 tensor-core (DMMA, mma.sync m16n8k4 .f64) fragment helpers;
-//   * exp(-dt K) application: dense (DMMA) and separable (A (x) A circulant) forms;
+//   * the dense (DMMA) exp(-dt K) application;
 //   * block reductions.
 #pragma once
 #include <cuda_runtime.h>
@@ -136,114 +136,6 @@ __device__ inline void atomic_max_double(double* addr, double val) {
     if (__longlong_as_double(assumed) >= val) return;
     old = atomicCAS(p, assumed, __double_as_longlong(val));
   } while (old != assumed);
-}
-
-// ------------------------------------------------------------------------------------
-//  Separable exp(-dt K): for the uniform NN hopping on the L x L torus,
-//    exp(-dt K) = exp(dt mu) * A (x) A,   A = exp(dt t H_1d) circulant, A[x][x'] = a[(x-x') mod L],
-//  with site index i = x + L y (src/square_lattice.cpp:30-61). Applied to a matrix M with
-//  leading dimension ld in two in-place passes of length-L circular convolutions.
-//  side 0: M <- c (A(x)A) M  (rows);  side 1: M <- c M (A(x)A)  (columns).
-//  rows/cols outside [0, N) are untouched. All threads of the block participate.
-// ------------------------------------------------------------------------------------
-// SC selects an optional diagonal scaling fused into the pass: element (i, j) is multiplied by
-// (s[i] > 0 ? rp : rm) * (s[j] > 0 ? cp : cm), on load (SC = 1, before the convolution) or
-// on store (SC = 2); SC = 0 leaves the pass unscaled
-// MEAS = 1 / 2 also accumulates the equal-time estimator sums of the matrix as loaded /
-// as stored (mtr, mdd, msq; see measure_commit)
-template <int L, int SC, int MEAS = 0>
-__device__ __forceinline__ void sep_pass(double* M, int ld, int N, const double* __restrict__ coef, double c, int side,
-                                int pass, const int8_t* sf, double rp, double rm, double cp, double cm,
-                                double& mtr, double& mdd, double& msq) {
-  // circulant coefficients in registers (compile-time indices after unrolling)
-  double a[L];
-#pragma unroll
-  for (int d = 0; d < L; ++d) a[d] = coef[d];
-  const int nfib = N * L;  // N lines (columns for side 0, rows for side 1) x L fibers each
-  for (int f = threadIdx.x; f < nfib; f += blockDim.x) {
-    const int line = f % N;   // column j (side 0) or row i (side 1)
-    const int o = f / N;      // the fixed lattice coordinate of the fiber
-    // pass 0 runs over x with y = o (sites L*o + e); pass 1 over y with x = o (sites o + L*e)
-    const int base_site = (pass == 0) ? (L * o) : o;
-    const int step_site = (pass == 0) ? 1 : L;
-    double* base = (side == 0) ? (M + base_site + (size_t)line * ld) : (M + line + (size_t)base_site * ld);
-    const size_t stride = (side == 0) ? (size_t)step_site : (size_t)step_site * ld;
-    // the factor of element e is (row factor) * (column factor); side 0: the line is column
-    // j and the site row i; side 1: the line is row i and the site column j
-    double lf = 1.0, sp = 1.0, sm = 1.0;
-    if (SC) {
-      const bool lpos = sf[line] > 0;
-      lf = (side == 0) ? (lpos ? cp : cm) : (lpos ? rp : rm);
-      sp = (side == 0) ? rp : cp;
-      sm = (side == 0) ? rm : cm;
-    }
-    double v[L];
-#pragma unroll
-    for (int e = 0; e < L; ++e) {
-      v[e] = base[e * stride];
-      if (MEAS == 1) {
-        msq = fma(v[e], v[e], msq);
-        if (base_site + e * step_site == line) { mtr += v[e]; mdd += (1.0 - v[e]) * (1.0 - v[e]); }
-      }
-      if (SC == 1) {
-        const double sfac = sf[base_site + e * step_site] > 0 ? sp : sm;
-        v[e] *= (side == 0) ? sfac * lf : lf * sfac;
-      }
-    }
-    // L independent accumulators, each summed over e2 in ascending order
-    double acc[L];
-#pragma unroll
-    for (int e = 0; e < L; ++e) acc[e] = 0.0;
-#pragma unroll
-    for (int e2 = 0; e2 < L; ++e2) {
-#pragma unroll
-      for (int e = 0; e < L; ++e) acc[e] = fma(a[(e - e2 + L) % L], v[e2], acc[e]);
-    }
-#pragma unroll
-    for (int e = 0; e < L; ++e) {
-      double out = (pass == 1) ? acc[e] * c : acc[e];
-      if (SC == 2) {
-        const double sfac = sf[base_site + e * step_site] > 0 ? sp : sm;
-        out *= (side == 0) ? sfac * lf : lf * sfac;
-      }
-      if (MEAS == 2) {
-        msq = fma(out, out, msq);
-        if (base_site + e * step_site == line) { mtr += out; mdd += (1.0 - out) * (1.0 - out); }
-      }
-      base[e * stride] = out;
-    }
-  }
-}
-
-// both passes of one side; SC0 / SC1 select the fused scaling of pass 0 / pass 1, M0 / M1
-// the fused estimators of pass 0 / pass 1 (added to acc_meas)
-template <int L, int SC0 = 0, int SC1 = 0, int M0 = 0, int M1 = 0>
-__device__ __forceinline__ void sep_apply(double* M, int ld, int N, const double* a, double c, int side,
-                                 const int8_t* sf = nullptr, double rp = 1.0, double rm = 1.0, double cp = 1.0,
-                                 double cm = 1.0, double* acc_meas = nullptr, double* red = nullptr) {
-  double mtr = 0.0, mdd = 0.0, msq = 0.0;
-  sep_pass<L, SC0, M0>(M, ld, N, a, c, side, 0, sf, rp, rm, cp, cm, mtr, mdd, msq);
-  __syncthreads();
-  sep_pass<L, SC1, M1>(M, ld, N, a, c, side, 1, sf, rp, rm, cp, cm, mtr, mdd, msq);
-  __syncthreads();
-  if (M0 || M1) measure_commit(mtr, mdd, msq, N, acc_meas, red);
-}
-
-// dispatch on the lattice size to an exact compile-time fiber length (L <= HQ_MAX_L)
-template <int SC0 = 0, int SC1 = 0, int M0 = 0, int M1 = 0>
-__device__ __forceinline__ void sep_apply_any(double* M, int ld, int N, int L, const double* a, double c, int side,
-                                     const int8_t* sf = nullptr, double rp = 1.0, double rm = 1.0,
-                                     double cp = 1.0, double cm = 1.0, double* acc_meas = nullptr,
-                                     double* red = nullptr) {
-  switch (L) {
-#define HQ_SEP_CASE(n) \
-  case n: sep_apply<n, SC0, SC1, M0, M1>(M, ld, N, a, c, side, sf, rp, rm, cp, cm, acc_meas, red); break;
-    HQ_SEP_CASE(1) HQ_SEP_CASE(2) HQ_SEP_CASE(3) HQ_SEP_CASE(4) HQ_SEP_CASE(5) HQ_SEP_CASE(6)
-    HQ_SEP_CASE(7) HQ_SEP_CASE(8) HQ_SEP_CASE(9) HQ_SEP_CASE(10) HQ_SEP_CASE(11) HQ_SEP_CASE(12)
-    HQ_SEP_CASE(13) HQ_SEP_CASE(14) HQ_SEP_CASE(15)
-#undef HQ_SEP_CASE
-    default: sep_apply<16, SC0, SC1, M0, M1>(M, ld, N, a, c, side, sf, rp, rm, cp, cm, acc_meas, red); break;
-  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -380,30 +272,6 @@ __device__ inline void dense_apply_right(double* M, int ld, int N, const double*
       }
     }
     __syncthreads();
-  }
-}
-
-// M <- diag(v) M (rows) with v_i = (s_i > 0 ? vp : vm) ; fields is the slice's int8 row
-__device__ inline void scale_rows(double* M, int ld, int N, const int8_t* s, double vp, double vm) {
-  HQ_FOR_EACH_ELEM(N, i, j) M[i + (size_t)j * ld] *= (s[i] > 0 ? vp : vm);
-}
-// M <- M diag(v) (columns)
-__device__ inline void scale_cols(double* M, int ld, int N, const int8_t* s, double vp, double vm) {
-  HQ_FOR_EACH_ELEM(N, i, j) M[i + (size_t)j * ld] *= (s[j] > 0 ? vp : vm);
-}
-
-// M <- expK M   (side 0)  /  M <- M expK (side 1); inv selects inv_expK
-__device__ inline void apply_expk(const HqChain& ch, double* M, int ld, int side, bool inv, double* stage) {
-  if (ch.expk_mode == HQK_EXPK_SEPARABLE) {
-#ifndef HQ_TEST_NO_SEP
-    sep_apply_any(M, ld, ch.N, ch.L, inv ? ch.sep_ai : ch.sep_a, inv ? ch.sep_ci : ch.sep_c, side);
-#endif
-  } else {
-#ifndef HQ_TEST_NO_DENSE
-    const double* E = inv ? ch.inv_expK : ch.expK;
-    if (side == 0) dense_apply(M, ld, ch.N, E, stage);
-    else dense_apply_right(M, ld, ch.N, E, stage);
-#endif
   }
 }
 

@@ -21,7 +21,8 @@ k_interval(const HqChain* __restrict__ chains, int nchains, int dir, int b, int 
   }
   __syncthreads();
   if (!ch.active || b >= ch.n_stab) return;
-  interval_body(ch, dir, b, flags, resident != 0, smem, sc, 0u);
+  if (resident) interval_body<true>(ch, dir, b, flags, smem, sc, 0u);
+  else interval_body<false>(ch, dir, b, flags, smem, sc, 0u);
 }
 
 cudaError_t launch_interval(const HqChain* chains, int n, int dir, int b, int flags, int Nmax, int kmax, bool resident,

@@ -9,140 +9,133 @@
 
 namespace hq {
 
-template <int NB>
-__device__ __forceinline__ void metropolis_slice_blk(const HqChain& ch, double* G, int ld, const MetroShared& sh, uint32_t& rng,
-                                     double& n_acc, int flags, long long log_base) {
-  const int N = ch.N;
-  const int ldp = panel_ld(N);
+// the interval body's shared-memory words of chain size N (see IntervalLayout)
+__device__ __forceinline__ MetroShared metro_shared(double* smem, const IntervalLayout& o, int N) {
+  MetroShared sh;
+  sh.X = smem + o.work;
+  sh.Y = smem + o.Y;
+  sh.xt = smem + o.rec;
+  sh.yt = sh.xt + 16 * kLdR;
+  sh.qg = sh.yt + 16 * kLdR;
+  sh.dl = smem + o.dl;
+  sh.thr = smem + o.thr;
+  sh.u = smem + o.u;
+  sh.rr = smem + o.rr;
+  sh.s = reinterpret_cast<int8_t*>(smem + o.fields);
+  sh.flip = sh.s + N;
+  sh.pw = reinterpret_cast<uint32_t*>(smem + o.pw);
+  sh.ired = reinterpret_cast<int*>(smem + o.ints);
+  sh.qj = sh.ired + 4;
+  return sh;
+}
+
+// The Metropolis visits of one slice's N sites (see hq_metropolis.cuh) from the random state rng;
+// returns the accepted flips (thread 0). L > 0: G in shared memory in the padded layout
+// (interval_ld, tile_cols) of the lattice size L; L = 0: G in global memory, any N, checked against
+// the edge. NB = the chain's delay depth: sites per block (4, 8 or 16). Every thread calls it. A
+// function of its own per lattice size: registers and code of one size do not weigh on the others.
+template <int L>
+__device__ __noinline__ int metropolis_slice(const HqChain& ch, uint32_t rng, int flags, long long log_base) {
+  extern __shared__ __align__(16) double smem[];
+  const int N = L > 0 ? L * L : ch.N;
+  const IntervalLayout lay = interval_layout(N, L > 0 ? 16 : ch.kmax, L > 0);
+  const MetroShared sh = metro_shared(smem, lay, N);
+  double* G = L > 0 ? smem + lay.G : ch.G;
+  const int ld = L > 0 ? interval_ld(N) : N;
+  const int ldp = panel_ld(pad16(N));
+  const int NB = ch.kmax;
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool log = (flags & HQ_F_LOG_RATIOS) && ch.ratios;
   // uniforms of this slice: site i consumes engine draws 2i+1, 2i+2 after the current state
   for (int i = tid; i < N; i += blockDim.x) {
     const uint32_t x1 = minstd_mulmod(sh.pw[i], rng);
     const uint32_t x2 = minstd_mulmod(kMinstdA, x1);
-    sh.u[i] = canonical_from_pair(x1, x2);
-    sh.dl[i] = sh.s[i] > 0 ? ch.delta_p : ch.delta_m;
-    sh.flip[i] = 0;
+    const double u = canonical_from_pair(x1, x2), dl = sh.s[i] > 0 ? ch.delta_p : ch.delta_m;
+    sh.u[i] = u;
+    sh.dl[i] = dl;
+    sh.thr[i] = u * (1.0 + dl);
   }
-  rng = minstd_mulmod(minstd_pow(2ull * N), rng);
   __syncthreads();
-  double acc_count = 0.0;
+  int acc_count = 0;
   for (int b0 = 0, bi = 0; b0 < N; b0 += NB, ++bi) {
-    if (warp == 0) {
-      const int nb = min(NB, N - b0);
-      // the fast walk without the ratio log unless it is on; near a tie the exact walk again
-      if constexpr (NB == 16) {
-        const bool near = log ? walk_block16<false, true>(ch, G, ld, sh, b0, nb, true, bi & 1)
-                              : walk_block16<false, false>(ch, G, ld, sh, b0, nb, false, bi & 1);
-        if (near) walk_block16<true>(ch, G, ld, sh, b0, nb, log, bi & 1);
-      } else {
-        const bool near = log ? walk_block<NB, false, true>(ch, G, ld, sh, b0, nb, true, bi & 1)
-                              : walk_block<NB, false, false>(ch, G, ld, sh, b0, nb, false, bi & 1);
-        if (near) walk_block<NB, true>(ch, G, ld, sh, b0, nb, log, bi & 1);
-      }
-    }
+    if (warp == 0) walk(G, ld, sh, b0, min(NB, N - b0), log, bi & 1);
     __syncthreads();
     // the count alternates between two words: with no flush (a == 0) no barrier follows,
     // and warp 0 writes the next block's count while other warps may still read this one
     const int a = sh.ired[bi & 1];
-    if (tid == 0) acc_count += a;
+    acc_count += a;
     if (a == 0) continue;
-    build_panels<NB>(G, ld, N, sh, ldp, a, b0);
-    __syncthreads();
-    flush_block(G, ld, N, sh.X, ldp, sh.Y, ldp, a);
+    for_ksteps(a, [&](auto kc) {
+      constexpr int KA = decltype(kc)::value;
+      build_panels<KA>(G, ld, N, sh, ldp, a, b0);
+      __syncthreads();
+      if constexpr (L > 0) rank_strips<pad16(L * L) / 16, tile_cols(L * L), KA>(G, ld, sh, ldp, ldp);
+    });
+    if constexpr (L == 0) rank_update48(G, ld, N, N, sh, ldp, ldp, a);
     __syncthreads();
   }
-  __syncthreads();
-  n_acc += acc_count;
   // apply the flips of this slice and optionally log the visit-time ratios
   for (int i = tid; i < N; i += blockDim.x) {
     if (sh.flip[i]) sh.s[i] = -sh.s[i];
     if (log && log_base + i < ch.ratio_cap) ch.ratios[log_base + i] = sh.rr[i];
   }
   __syncthreads();
+  return acc_count;
+}
+template <bool RES>
+__device__ __forceinline__ int metropolis_dispatch(const HqChain& ch, uint32_t rng, int flags, long long log_base) {
+  int a = 0;
+  if constexpr (RES) {
+    for_lattice(ch.L, [&](auto lc) {
+      constexpr int L = decltype(lc)::value;
+      if constexpr (L <= 12) a = metropolis_slice<L>(ch, rng, flags, log_base);
+    });
+  } else {
+    a = metropolis_slice<0>(ch, rng, flags, log_base);
+  }
+  return a;
 }
 
-// block size NB of the submatrix updates: the chain's delay depth (4, 8 or 16)
-__device__ __forceinline__ void metropolis_dispatch(const HqChain& ch, double* G, int ld, const MetroShared& sh, uint32_t& rng,
-                                    double& n_acc, int flags, long long log_base) {
-  if (ch.kmax >= 16) metropolis_slice_blk<16>(ch, G, ld, sh, rng, n_acc, flags, log_base);
-  else if (ch.kmax >= 8) metropolis_slice_blk<8>(ch, G, ld, sh, rng, n_acc, flags, log_base);
-  else metropolis_slice_blk<4>(ch, G, ld, sh, rng, n_acc, flags, log_base);
-}
-
-// Shared-memory words of the interval body besides its dynamic region (interval_smem_doubles):
-// reductions, block counts, the barrier of the bulk load of G and the walk records.
+// Shared-memory words of the interval body besides its dynamic region: reductions and the barrier
+// of the bulk load of G (initialised for one arrival).
 struct IntervalScratch {
   double* red;     // 96 doubles
-  int* ired;       // 64 ints
-  uint64_t* gbar;  // mbarrier of the bulk load of G (initialised for one arrival)
-  int* qj;         // 16 ints
-  double* qg;      // 16 doubles
-  double* xt;      // 16 x 16 doubles, 16-byte aligned
-  double* yt;      // 16 x 16 doubles, 16-byte aligned
+  uint64_t* gbar;
 };
-constexpr int kIntervalScratchBytes = (96 + 16 + 512) * 8 + (64 + 16) * 4 + 16;
+constexpr int kIntervalScratchBytes = (96 + 2) * 8;
 
 // Places the interval scratch at `p` (16-byte aligned, kIntervalScratchBytes long).
 __device__ __forceinline__ IntervalScratch interval_scratch_at(void* p) {
-  IntervalScratch sc;
   double* d = reinterpret_cast<double*>(p);
-  sc.xt = d; d += 256;
-  sc.yt = d; d += 256;
-  sc.red = d; d += 96;
-  sc.qg = d; d += 16;
-  sc.gbar = reinterpret_cast<uint64_t*>(d); d += 2;
-  sc.ired = reinterpret_cast<int*>(d);
-  sc.qj = sc.ired + 64;
-  return sc;
+  return {d, reinterpret_cast<uint64_t*>(d + 96)};
 }
 
 // The update (or no-update) slices of stabilisation interval b of chain `ch` in direction dir.
-// `smem` is the dynamic region (interval_smem_doubles(N, kmax, resident) doubles); gpar is the
+// `smem` is the block's dynamic shared memory (interval_smem_doubles(N, kmax, RES) doubles); gpar is the
 // phase parity of sc.gbar for this interval's bulk load of G. Every thread of the block calls
 // it; the chain is active and b < n_stab.
-__device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b, int flags, bool resident, double* smem,
+template <bool RES>
+__device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b, int flags, double* smem,
                                               const IntervalScratch& sc, unsigned gpar) {
   const int N = ch.N;
   int t_lo, t_hi;
   interval_range(ch.nt, ch.pace, ch.n_stab, dir, b, t_lo, t_hi);
 
-  // shared-memory carve-up; the resident G moves in and out by bulk copies of its columns
-  // (cp.async per element where the columns are not 16-byte multiples)
-  double* p = smem;
-  double* G;
-  int ld;
+  // the resident G moves in and out by bulk copies of its columns (cp.async per element where the
+  // columns are not 16-byte multiples)
+  const IntervalLayout lay = interval_layout(N, ch.kmax, RES);
+  double* G = RES ? smem + lay.G : ch.G;
+  const int ld = RES ? interval_ld(N) : N;
   bool bulk = false;
-  if (resident) {
-    G = p;
-    ld = interval_ld(N);
-    p += (size_t)N * ld;
+  if (RES) {
     bulk = bulk_columns_ok(ch.G, N, ld);
     if (bulk) load_mat_bulk(G, ld, ch.G, N, sc.gbar, ch.acc + HQ_ACC_STATUS, gpar);
     else load_mat_async(G, ld, ch.G, N, N);
-  } else {
-    G = ch.G;
-    ld = N;
   }
-  const size_t panels = (size_t)panel_ld(N) * ch.kmax * 2;
-  const size_t stage_n = (size_t)8 * (((N + 15) & ~15) + 4);
-  double* work = p;
-  p += panels > stage_n ? panels : stage_n;
-  MetroShared sh;
-  sh.X = work;
-  sh.Y = work + (size_t)panel_ld(N) * ch.kmax;
-  sh.dl = p; p += N;
-  sh.u = p; p += N;
-  sh.rr = p; p += N;
-  sh.s = reinterpret_cast<int8_t*>(p);
-  sh.flip = sh.s + N;
-  sh.pw = reinterpret_cast<uint32_t*>(p + (N + 7) / 4);
+  const MetroShared sh = metro_shared(smem, lay, N);
+  double *work = sh.X, *vp = smem + lay.vp, *vm = smem + lay.vm;
   for (int i = threadIdx.x; i < N; i += blockDim.x) sh.pw[i] = minstd_pow(2ull * i + 1);
-  sh.ired = sc.ired;
-  sh.qj = sc.qj;
-  sh.qg = sc.qg;
-  sh.xt = sc.xt;
-  sh.yt = sc.yt;
+  const uint64_t slice_jump = minstd_pow(2ull * N);  // the engine's state after a slice's 2 N draws
   uint32_t rng = *ch.rng;
   double n_acc = 0.0, n_prop = 0.0;
   long long log_base = (flags & HQ_F_LOG_RATIOS) && ch.ratio_count ? *ch.ratio_count : 0;
@@ -152,25 +145,28 @@ __device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b,
   // up / down sweeps in separable mode measure inside the wrap (up: slice t's G in the wrap of
   // slice t+1; down: in the wrap of slice t itself); the last slice of the interval is
   // measured after stabilisation
-  const bool fused = (flags & HQ_F_MEASURE) && ch.expk_mode == HQK_EXPK_SEPARABLE &&
+  const bool fused = (flags & HQ_F_MEASURE) && ch.expk_mode == HQK_EXPK_SEPARABLE && wrap_measures<RES>(ch.L) &&
                      (dir == HQ_UP || dir == HQ_DOWN);
   for (int step = 0; step < nsl; ++step) {
     const int t = (dir == HQ_DOWN) ? (t_hi - step) : (t_lo + step);
     const int l = t % ch.nt;
     for (int i = threadIdx.x; i < N; i += blockDim.x) sh.s[i] = ch.fields[(size_t)l * N + i];
     __syncthreads();
-    if (dir == HQ_UP) {
-      wrap_slice(ch, G, ld, sh.s, HQ_UP, work, (fused && step > 0) ? ch.acc : nullptr, sc.red);
-      metropolis_dispatch(ch, G, ld, sh, rng, n_acc, flags, log_base);
+    if (dir != HQ_DOWN) {
+      slice_factors(ch, sh.s, vp, vm);
+      __syncthreads();
+      wrap_slice<RES>(ch, G, ld, vp, vm, HQ_UP, work, (fused && step > 0) ? ch.acc : nullptr, sc.red);
+    }
+    if (dir == HQ_UP || dir == HQ_DOWN) {
+      n_acc += metropolis_dispatch<RES>(ch, rng, flags, log_base);
+      rng = minstd_mulmod(slice_jump, rng);
       n_prop += N;
       log_base += N;
-    } else if (dir == HQ_DOWN) {
-      metropolis_dispatch(ch, G, ld, sh, rng, n_acc, flags, log_base);
-      n_prop += N;
-      log_base += N;
-      wrap_slice(ch, G, ld, sh.s, HQ_DOWN, work, (fused && step < nsl - 1) ? ch.acc : nullptr, sc.red);
-    } else {
-      wrap_slice(ch, G, ld, sh.s, HQ_UP, work);
+    }
+    if (dir == HQ_DOWN) {
+      slice_factors(ch, sh.s, vp, vm);
+      __syncthreads();
+      wrap_slice<RES>(ch, G, ld, vp, vm, HQ_DOWN, work, (fused && step < nsl - 1) ? ch.acc : nullptr, sc.red);
     }
     for (int i = threadIdx.x; i < N; i += blockDim.x) ch.fields[(size_t)l * N + i] = sh.s[i];
     if (step < nsl - 1) {
@@ -180,7 +176,7 @@ __device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b,
     }
     __syncthreads();
   }
-  if (resident) {
+  if (RES) {
     if (bulk) store_mat_bulk(ch.G, G, ld, N);
     else copy_mat(ch.G, N, G, ld, N);
   }

@@ -37,7 +37,7 @@ constexpr int kNE = kNC / kL;              // y values (x-fibres) of the column 
 }  // namespace
 
 __host__ __device__ inline size_t interval_cl_smem_doubles() {
-  return (size_t)kNC * kLd + (size_t)kLdx * 16 + (size_t)16 * kLdy + 3 * kNC + kNC / 2 + (kN + kNC + 7) / 8 + 16;
+  return (size_t)kNC * kLd + (size_t)kLdx * 16 + (size_t)16 * kLdy + 4 * kNC + 2 * kN + kNC / 2 + (kN + kNC + 7) / 8 + 16;
 }
 size_t smem_interval_cl_bytes() { return interval_cl_smem_doubles() * sizeof(double); }
 
@@ -45,78 +45,21 @@ bool interval_cluster_ok(int N, int L, int expk_mode, int kmax) {
   return N == kN && L == kL && expk_mode == HQK_EXPK_SEPARABLE && kmax == 16;
 }
 
-// One local pass of the separable exp(-dt K) on this CTA's columns (side 0: along the rows of
-// every local column; side 1, pass 0: along x inside the rows' local y values). The same
-// arithmetic as sep_pass (scaling on load / store, L accumulators summed in ascending order).
-template <int SIDE, int PASS, int SC>
-__device__ __forceinline__ void cl_local_pass(double* Gc, int c0, const double* __restrict__ coef, double cmul,
-                                              const int8_t* sf, double rp, double rm, double cp, double cm) {
-  static_assert(SIDE == 0 || PASS == 0, "the column-side y-pass exchanges data");
+// The y-pass of the column side (M <- c M (1 (x) A) along y; SC = 2 multiplies element (i, j) by
+// sl[i] sc[j] on store): the fibre of row i and x = o holds the columns o + 16 e, e = 0..15, four in
+// each CTA; this CTA's outputs are e = ELO .. ELO + 3. Rows are taken 16 at a time (one fibre per
+// thread): every thread reads its fibre's 16 inputs (12 of them from the other CTAs), the cluster
+// barrier lets every CTA finish reading, then each CTA writes its own 4 outputs. ELO is a
+// compile-time value so that the rotated coefficients stay in registers (a runtime rotation reads
+// 64 of them from shared memory per fibre).
+template <int SC, int ELO>
+__device__ __forceinline__ void cl_exchange_pass(double* Gc, double* const* Gr, const double* coef, double c, const double* sc,
+                                                 const double* sl, cg::cluster_group& cluster) {
+  constexpr int rows_per_chunk = HQ_INT_THREADS / kL;
   double a[kL];
 #pragma unroll
   for (int d = 0; d < kL; ++d) a[d] = coef[d];
-  // side 0: lines = local columns (kNC), fibres per line: kL (o); side 1: lines = rows (kN), o = local y
-  constexpr int nfib = (SIDE == 0) ? kNC * kL : kN * kNE;
-  for (int f = threadIdx.x; f < nfib; f += blockDim.x) {
-    int line, o;
-    if (SIDE == 0) { line = f % kNC; o = f / kNC; } else { line = f % kN; o = c0 / kL + f / kN; }
-    const int base_site = (SIDE == 0 && PASS == 1) ? o : kL * o;
-    const int step_site = (SIDE == 0 && PASS == 1) ? kL : 1;
-    double* base;
-    size_t stride;
-    if (SIDE == 0) { base = Gc + base_site + (size_t)line * kLd; stride = (size_t)step_site; }
-    else { base = Gc + line + (size_t)(base_site - c0) * kLd; stride = (size_t)kLd; }
-    const int line_site = (SIDE == 0) ? c0 + line : line;
-    double lf = 1.0, sp = 1.0, sm = 1.0;
-    if (SC) {
-      const bool lpos = sf[line_site] > 0;
-      lf = (SIDE == 0) ? (lpos ? cp : cm) : (lpos ? rp : rm);
-      sp = (SIDE == 0) ? rp : cp;
-      sm = (SIDE == 0) ? rm : cm;
-    }
-    double v[kL];
-#pragma unroll
-    for (int e = 0; e < kL; ++e) {
-      v[e] = base[e * stride];
-      if (SC == 1) {
-        const double sfac = sf[base_site + e * step_site] > 0 ? sp : sm;
-        v[e] *= (SIDE == 0) ? sfac * lf : lf * sfac;
-      }
-    }
-    double acc[kL];
-#pragma unroll
-    for (int e = 0; e < kL; ++e) acc[e] = 0.0;
-#pragma unroll
-    for (int e2 = 0; e2 < kL; ++e2) {
-#pragma unroll
-      for (int e = 0; e < kL; ++e) acc[e] = fma(a[(e - e2 + kL) % kL], v[e2], acc[e]);
-    }
-#pragma unroll
-    for (int e = 0; e < kL; ++e) {
-      double out = (PASS == 1) ? acc[e] * cmul : acc[e];
-      if (SC == 2) {
-        const double sfac = sf[base_site + e * step_site] > 0 ? sp : sm;
-        out *= (SIDE == 0) ? sfac * lf : lf * sfac;
-      }
-      base[e * stride] = out;
-    }
-  }
-}
-
-// The y-pass of the column side (M <- M (1 (x) A) along y, times cmul; SC = 2 scales on store
-// by row factor (rp / rm) x column factor (cp / cm)): the fibre of row i and x = o holds the
-// columns o + 16 e, e = 0..15, four in each CTA. Rows are taken 16 at a time (one fibre per
-// thread): every thread reads its fibre's 16 inputs (12 of them from the other CTAs), the
-// cluster barrier lets every CTA finish reading, then each CTA writes its own 4 outputs.
-// coef lives in the chain descriptor in shared memory: the rotation by this CTA's e_lo is a
-// runtime index, which a register array would turn into a local-memory one.
-template <int SC>
-__device__ __forceinline__ void cl_exchange_pass(double* Gc, double* const* Gr, int c0, const double* coef, double cmul,
-                                                 const int8_t* sf, double rp, double rm, double cp, double cm,
-                                                 cg::cluster_group& cluster) {
-  constexpr int rows_per_chunk = HQ_INT_THREADS / kL;
   const int o = threadIdx.x % kL;
-  const int e_lo = c0 / kL;  // this CTA's outputs: e = e_lo .. e_lo + kNE - 1
   for (int r0 = 0; r0 < kN; r0 += rows_per_chunk) {
     const int i = r0 + threadIdx.x / kL;
     double v[kL];
@@ -131,62 +74,72 @@ __device__ __forceinline__ void cl_exchange_pass(double* Gc, double* const* Gr, 
 #pragma unroll
     for (int e2 = 0; e2 < kL; ++e2) {
 #pragma unroll
-      for (int k = 0; k < kNE; ++k) acc[k] = fma(coef[(e_lo + k - e2 + kL) % kL], v[e2], acc[k]);
+      for (int k = 0; k < kNE; ++k) acc[k] = fma(a[(ELO + k - e2 + kL) % kL], v[e2], acc[k]);
     }
     cluster.sync();  // every CTA has read this chunk's rows
-    double lf = 1.0;
-    if (SC) lf = sf[i] > 0 ? rp : rm;
+    const double lf = SC == 2 ? sl[i] : 1.0;
 #pragma unroll
     for (int k = 0; k < kNE; ++k) {
-      const int j = o + kL * (e_lo + k);
-      double out = acc[k] * cmul;
-      if (SC == 2) {
-        const double sfac = sf[j] > 0 ? cp : cm;
-        out *= lf * sfac;
-      }
-      Gc[i + (size_t)(j - c0) * kLd] = out;
+      acc[k] *= c;
+      if (SC == 2) acc[k] *= lf * sc[o + kL * (ELO + k)];
+      Gc[i + (size_t)(o + kL * k) * kLd] = acc[k];
     }
   }
   __syncthreads();
 }
-
-// wrap of this CTA's columns by B(l) (the cluster form of wrap_slice's separable branch)
-__device__ __forceinline__ void cl_wrap(const HqChain& ch, double* Gc, double* const* Gr, int c0, const int8_t* s,
-                                        int dir, cg::cluster_group& cluster) {
-  if (dir == HQ_UP) {
-    // G <- e^V E G E^-1 e^-V: E on the rows, E^-1 on the columns with e^V / e^-V on the last pass's stores
-    cl_local_pass<0, 0, 0>(Gc, c0, ch.sep_a, ch.sep_c, s, 1.0, 1.0, 1.0, 1.0);
-    __syncthreads();
-    cl_local_pass<0, 1, 0>(Gc, c0, ch.sep_a, ch.sep_c, s, 1.0, 1.0, 1.0, 1.0);
-    __syncthreads();
-    cl_local_pass<1, 0, 0>(Gc, c0, ch.sep_ai, ch.sep_ci, s, 1.0, 1.0, 1.0, 1.0);
-    cluster.sync();  // the other CTAs' x-pass results are read next
-    cl_exchange_pass<2>(Gc, Gr, c0, ch.sep_ai, ch.sep_ci, s, ch.ev_p, ch.ev_m, ch.ev_m, ch.ev_p, cluster);
-  } else {
-    // G <- E^-1 e^-V G e^V E: the scalings on the first pass's loads
-    cl_local_pass<0, 0, 1>(Gc, c0, ch.sep_ai, ch.sep_ci, s, ch.ev_m, ch.ev_p, ch.ev_p, ch.ev_m);
-    __syncthreads();
-    cl_local_pass<0, 1, 0>(Gc, c0, ch.sep_ai, ch.sep_ci, s, 1.0, 1.0, 1.0, 1.0);
-    __syncthreads();
-    cl_local_pass<1, 0, 0>(Gc, c0, ch.sep_a, ch.sep_c, s, 1.0, 1.0, 1.0, 1.0);
-    cluster.sync();
-    cl_exchange_pass<0>(Gc, Gr, c0, ch.sep_a, ch.sep_c, s, 1.0, 1.0, 1.0, 1.0, cluster);
+template <int SC>
+__device__ __forceinline__ void cl_exchange(double* Gc, double* const* Gr, int rank, const double* coef, double c,
+                                            const double* sc, const double* sl, cg::cluster_group& cluster) {
+  static_assert(kNE == 4 && kCl == 4, "one case per CTA of the cluster");
+  switch (rank) {
+    case 0: cl_exchange_pass<SC, 0>(Gc, Gr, coef, c, sc, sl, cluster); break;
+    case 1: cl_exchange_pass<SC, 4>(Gc, Gr, coef, c, sc, sl, cluster); break;
+    case 2: cl_exchange_pass<SC, 8>(Gc, Gr, coef, c, sc, sl, cluster); break;
+    default: cl_exchange_pass<SC, 12>(Gc, Gr, coef, c, sc, sl, cluster); break;
   }
 }
 
-// Metropolis over the N sites of the slice (see the one-CTA metropolis_slice_blk): the owner
-// of each 16-site block walks it; X by the owner, Y and the flush by every CTA.
-__device__ __forceinline__ void cl_metropolis(const HqChain& ch, double* Gc, int rank, int c0, MetroShared& sh,
-                                              double* u_l, double* dl_l, int8_t* flip_l, const uint32_t* pw,
-                                              double* Xl, double* Yl, uint32_t& rng, double& n_acc, bool log,
-                                              cg::cluster_group& cluster) {
+// wrap of this CTA's columns by B(l) (the cluster form of wrap_slice's separable branch); vp = e^V,
+// vm = e^-V of all N sites
+__device__ __forceinline__ void cl_wrap(const HqChain& ch, double* Gc, double* const* Gr, int rank, const double* vp,
+                                        const double* vm, int dir, cg::cluster_group& cluster) {
+  const int c0 = rank * kNC;
+  SepMeas ms;
+  double a[kL];
+  if (dir == HQ_UP) {
+    // G <- e^V E G E^-1 e^-V: E on the rows, E^-1 on the columns with e^V / e^-V on the last pass's stores
+    sep_side<kL, kLd, 0, 0, 0, kNC>(Gc, kLd, ch.sep_a, ch.sep_c, nullptr, nullptr, ms);
+#pragma unroll
+    for (int d = 0; d < kL; ++d) a[d] = ch.sep_ai[d];
+    sep_pass<kL, kLd, 1, 0, 0, 0, kNC>(Gc, kLd, a, 1.0, nullptr, nullptr, ms);
+    cluster.sync();  // the other CTAs' x-pass results are read next
+    cl_exchange<2>(Gc, Gr, rank, ch.sep_ai, ch.sep_ci, vm, vp, cluster);
+  } else {
+    // G <- E^-1 e^-V G e^V E: the scalings on the first pass's loads
+    sep_side<kL, kLd, 0, 1, 0, kNC>(Gc, kLd, ch.sep_ai, ch.sep_ci, vm, vp + c0, ms);
+#pragma unroll
+    for (int d = 0; d < kL; ++d) a[d] = ch.sep_a[d];
+    sep_pass<kL, kLd, 1, 0, 0, 0, kNC>(Gc, kLd, a, 1.0, nullptr, nullptr, ms);
+    cluster.sync();
+    cl_exchange<0>(Gc, Gr, rank, ch.sep_a, ch.sep_c, nullptr, nullptr, cluster);
+  }
+}
+
+// Metropolis over the N sites of the slice (see the one-CTA metropolis_slice): the owner of each
+// 16-site block walks it and forms X from its own columns; every CTA forms Y for its own columns
+// from the walk's records, copies X from the owner through DSMEM and flushes its columns.
+__device__ __forceinline__ void cl_metropolis(const HqChain& ch, double* Gc, int rank, int c0, MetroShared& sh, double* u_l,
+                                              double* thr_l, double* dl_l, int8_t* flip_l, const uint32_t* pw,
+                                              uint32_t& rng, double& n_acc, bool log, cg::cluster_group& cluster) {
   const int tid = threadIdx.x, warp = tid >> 5;
   double* Gs = Gc - (size_t)c0 * kLd;  // absolute column index -> local storage
   for (int q = tid; q < kNC; q += blockDim.x) {
     const uint32_t x1 = minstd_mulmod(pw[q], rng);
     const uint32_t x2 = minstd_mulmod(kMinstdA, x1);
-    u_l[q] = canonical_from_pair(x1, x2);
-    dl_l[q] = sh.s[c0 + q] > 0 ? ch.delta_p : ch.delta_m;
+    const double u = canonical_from_pair(x1, x2), dl = sh.s[c0 + q] > 0 ? ch.delta_p : ch.delta_m;
+    u_l[q] = u;
+    dl_l[q] = dl;
+    thr_l[q] = u * (1.0 + dl);
     flip_l[q] = 0;
   }
   rng = minstd_mulmod(minstd_pow(2ull * kN), rng);
@@ -195,86 +148,36 @@ __device__ __forceinline__ void cl_metropolis(const HqChain& ch, double* Gc, int
   for (int b0 = 0, bi = 0; b0 < kN; b0 += 16, ++bi) {
     const int owner = b0 / kNC;
     const int slot = bi & 1;
-    if (rank == owner && warp == 0) {
-      const bool near = log ? walk_block16<false, true>(ch, Gs, kLd, sh, b0, 16, true, slot)
-                            : walk_block16<false, false>(ch, Gs, kLd, sh, b0, 16, false, slot);
-      if (near) walk_block16<true>(ch, Gs, kLd, sh, b0, 16, log, slot);
-    }
+    if (rank == owner && warp == 0) walk(Gs, kLd, sh, b0, 16, log, slot);
     cluster.sync();  // the walk's records are visible to the cluster
     const int* o_ired = cluster.map_shared_rank(sh.ired, owner);
     const int a = o_ired[slot];
     if (rank == owner && tid == 0) acc_count += a;
     if (a == 0) continue;
     if (rank != owner) {
-      const double* oxt = cluster.map_shared_rank(sh.xt, owner);
-      const double* oyt = cluster.map_shared_rank(sh.yt, owner);
+      const double* orec = cluster.map_shared_rank(sh.xt, owner);
       const int* oqj = cluster.map_shared_rank(sh.qj, owner);
-      const double* oqg = cluster.map_shared_rank(sh.qg, owner);
-      for (int k = tid; k < 256; k += blockDim.x) { sh.xt[k] = oxt[k]; sh.yt[k] = oyt[k]; }
-      if (tid < 16) { sh.qj[tid] = oqj[tid]; sh.qg[tid] = oqg[tid]; }
+      for (int k = tid; k < kRecordDoubles; k += blockDim.x) sh.xt[k] = orec[k];
+      if (tid < 16) sh.qj[tid] = oqj[tid];
       __syncthreads();
     }
-    // the owner: X[p, m] = gamma_m (G[p, j_m] + sum_{m'<m} X[p, m'] Y[m', j_m]) for every row p
-    if (rank == owner) {
-      for (int p = tid; p < kN; p += blockDim.x) {
-        double x[16];
+    for_ksteps(a, [&](auto kc) {
+      constexpr int KA = decltype(kc)::value;
+      if (tid >= 128) panel_cols<KA>(Gc + b0, kLd, kNC, c0, sh, a, b0, kLdy);
+      else if (rank == owner) panel_rows<KA>(Gs + (size_t)b0 * kLd, kLd, kN, sh, a, kLdx);
+      cluster.sync();  // X is complete in the owner's shared memory
+      if (rank != owner) {
+        const double* oX = cluster.map_shared_rank(sh.X, owner);
+        static_assert(HQ_INT_THREADS == kN, "one row of X per thread");
+        double v[4 * KA];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-          x[m] = 0.0;
-          if (m < a) {
-            const int jm = sh.qj[m], sj = jm - b0;
-            const double* cy = sh.yt + sj * 16;
-            double cx0 = Gs[p + (size_t)jm * kLd], cx1 = 0.0;
+        for (int m = 0; m < 4 * KA; ++m) v[m] = oX[tid + m * kLdx];
 #pragma unroll
-            for (int m2 = 0; m2 + 1 < m; m2 += 2) {
-              const double2 vy = *reinterpret_cast<const double2*>(cy + m2);
-              cx0 = fma(x[m2], vy.x, cx0);
-              cx1 = fma(x[m2 + 1], vy.y, cx1);
-            }
-            if (m & 1) cx0 = fma(x[m - 1], cy[m - 1], cx0);
-            x[m] = sh.qg[m] * (cx0 + cx1);
-          }
-        }
-#pragma unroll
-        for (int m = 0; m < 16; ++m)
-          if (m < a) Xl[p + m * kLdx] = x[m];
+        for (int m = 0; m < 4 * KA; ++m) sh.X[tid + m * kLdx] = v[m];
       }
-    }
-    // every CTA: Y[m, q] = G[j_m, q] - e_{j_m}(q) + sum_{m'<m} X[j_m, m'] Y[m', q] for its columns
-    for (int q = tid; q < kNC; q += blockDim.x) {
-      const int pc = c0 + q;
-      double y[16];
-#pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        y[m] = 0.0;
-        if (m < a) {
-          const int jm = sh.qj[m], sj = jm - b0;
-          const double* cx = sh.xt + sj * 16;
-          double cy0 = Gc[jm + (size_t)q * kLd] - (pc == jm ? 1.0 : 0.0), cy1 = 0.0;
-#pragma unroll
-          for (int m2 = 0; m2 + 1 < m; m2 += 2) {
-            const double2 vx = *reinterpret_cast<const double2*>(cx + m2);
-            cy0 = fma(vx.x, y[m2], cy0);
-            cy1 = fma(vx.y, y[m2 + 1], cy1);
-          }
-          if (m & 1) cy0 = fma(cx[m - 1], y[m - 1], cy0);
-          y[m] = cy0 + cy1;
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 16; ++m)
-        if (m < a) Yl[m * kLdy + q] = y[m];
-    }
-    cluster.sync();  // X is complete in the owner's shared memory
-    if (rank != owner) {
-      const double* oX = cluster.map_shared_rank(Xl, owner);
-      for (int k = tid; k < kN * a; k += blockDim.x) {
-        const int m = k / kN, p = k % kN;
-        Xl[p + m * kLdx] = oX[p + m * kLdx];
-      }
-    }
-    __syncthreads();
-    rank_update48(Gc, kLd, kN, kNC, Xl, kLdx, Yl, kLdy, a);
+      __syncthreads();
+      rank_strips<kN / 16, kNC / 8, KA>(Gc, kLd, sh, kLdx, kLdy);
+    });
     __syncthreads();
   }
   n_acc += acc_count;
@@ -294,10 +197,8 @@ k_interval_cl(const HqChain* __restrict__ chains, int nchains, int dir, int b, i
   __shared__ double part[2][3];  // this CTA's estimator partial sums, double-buffered by step
   __shared__ double acc_part;    // this CTA's accepted flips
   __shared__ int ired[4];
-  __shared__ int qj_s[16];
-  __shared__ double qg_s[16];
-  __shared__ __align__(16) double xt_s[16 * 16];
-  __shared__ __align__(16) double yt_s[16 * 16];
+  __shared__ __align__(16) int qj_s[16];
+  __shared__ __align__(16) double rec_s[kRecordDoubles];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int c = blockIdx.x / kCl;  // every CTA of a cluster serves the same chain
@@ -316,7 +217,10 @@ k_interval_cl(const HqChain* __restrict__ chains, int nchains, int dir, int b, i
   double* Yl = p; p += (size_t)16 * kLdy;
   double* u_l = p; p += kNC;
   double* dl_l = p; p += kNC;
+  double* thr_l = p; p += kNC;
   double* rr_l = p; p += kNC;
+  double* vp = p; p += kN;
+  double* vm = p; p += kN;
   uint32_t* pw = reinterpret_cast<uint32_t*>(p); p += kNC / 2;
   int8_t* s = reinterpret_cast<int8_t*>(p);
   int8_t* flip_l = s + kN;
@@ -330,18 +234,19 @@ k_interval_cl(const HqChain* __restrict__ chains, int nchains, int dir, int b, i
   for (int k = 0; k < kCl; ++k) Gr[k] = (k == rank) ? Gc : cluster.map_shared_rank(Gc, k);
   MetroShared sh;
   sh.dl = dl_l - c0;
+  sh.thr = thr_l - c0;
   sh.u = u_l - c0;
   sh.rr = rr_l - c0;
   sh.s = s;
   sh.flip = flip_l - c0;
   sh.X = Xl;
   sh.Y = Yl;
-  sh.xt = xt_s;
-  sh.yt = yt_s;
+  sh.xt = rec_s;
+  sh.yt = rec_s + 16 * kLdR;
+  sh.qg = rec_s + 32 * kLdR;
   sh.ired = ired;
   sh.pw = pw;
   sh.qj = qj_s;
-  sh.qg = qg_s;
   uint32_t rng = *ch.rng;
   const bool log = (flags & HQ_F_LOG_RATIOS) && ch.ratios;
   long long log_base = log && ch.ratio_count ? *ch.ratio_count : 0;
@@ -357,11 +262,15 @@ k_interval_cl(const HqChain* __restrict__ chains, int nchains, int dir, int b, i
     for (int i = threadIdx.x; i < kN; i += blockDim.x) s[i] = ch.fields[(size_t)l * kN + i];
     __syncthreads();
     if (dir == HQ_UP) {
-      cl_wrap(ch, Gc, Gr, c0, s, HQ_UP, cluster);
-      cl_metropolis(ch, Gc, rank, c0, sh, u_l, dl_l, flip_l, pw, Xl, Yl, rng, n_acc, log, cluster);
-    } else {
-      cl_metropolis(ch, Gc, rank, c0, sh, u_l, dl_l, flip_l, pw, Xl, Yl, rng, n_acc, log, cluster);
-      cl_wrap(ch, Gc, Gr, c0, s, HQ_DOWN, cluster);
+      slice_factors(ch, s, vp, vm);
+      __syncthreads();
+      cl_wrap(ch, Gc, Gr, rank, vp, vm, HQ_UP, cluster);
+    }
+    cl_metropolis(ch, Gc, rank, c0, sh, u_l, thr_l, dl_l, flip_l, pw, rng, n_acc, log, cluster);
+    if (dir == HQ_DOWN) {
+      slice_factors(ch, s, vp, vm);
+      __syncthreads();
+      cl_wrap(ch, Gc, Gr, rank, vp, vm, HQ_DOWN, cluster);
     }
     n_prop += kN;
     for (int q = threadIdx.x; q < kNC; q += blockDim.x) {
@@ -448,6 +357,8 @@ k_bchain_cols(const HqChain* __restrict__ chains, int nchains, int dir, int b) {
   const size_t NN = (size_t)kN * kN;
   double* Xc = smem;                      // kN x kNC, leading dimension kLd
   double* Dc = smem + (size_t)kNC * kLd;  // D of the stack top at the block's columns
+  double* v = Dc + kNC;                   // e^{V} of a slice
+  SepMeas ms;
   if (top >= 0) {
     const double* U = ch.stackU + ((size_t)side * ch.n_stab + top) * NN;
     const double* D = ch.stackD + ((size_t)side * ch.n_stab + top) * kN;
@@ -471,22 +382,16 @@ k_bchain_cols(const HqChain* __restrict__ chains, int nchains, int dir, int b) {
     for (int i = threadIdx.x; i < kN; i += blockDim.x) s[i] = ch.fields[(size_t)l * kN + i];
     __syncthreads();
     // e^{V} rides on the first pass (down: B^T = E e^V) or the last pass (up: B = e^V E)
-    if (dir == HQ_DOWN) {
-      cl_local_pass<0, 0, 1>(Xc, c0, ch.sep_a, ch.sep_c, s, ch.ev_p, ch.ev_m, 1.0, 1.0);
-      __syncthreads();
-      cl_local_pass<0, 1, 0>(Xc, c0, ch.sep_a, ch.sep_c, s, 1.0, 1.0, 1.0, 1.0);
-    } else {
-      cl_local_pass<0, 0, 0>(Xc, c0, ch.sep_a, ch.sep_c, s, 1.0, 1.0, 1.0, 1.0);
-      __syncthreads();
-      cl_local_pass<0, 1, 2>(Xc, c0, ch.sep_a, ch.sep_c, s, ch.ev_p, ch.ev_m, 1.0, 1.0);
-    }
+    slice_factors(ch, s, v, nullptr);
     __syncthreads();
+    if (dir == HQ_DOWN) sep_side<kL, kLd, 0, 1, 0, kNC>(Xc, kLd, ch.sep_a, ch.sep_c, v, nullptr, ms);
+    else sep_side<kL, kLd, 0, 2, 0, kNC>(Xc, kLd, ch.sep_a, ch.sep_c, v, nullptr, ms);
   }
   for (int j = threadIdx.x >> 5; j < kNC; j += blockDim.x >> 5)
     for (int i = threadIdx.x & 31; i < kN; i += 32) ch.X[i + (size_t)(c0 + j) * kN] = Xc[i + (size_t)j * kLd];
 }
 
-size_t smem_bchain_cols_bytes() { return ((size_t)kNC * kLd + kNC) * sizeof(double); }
+size_t smem_bchain_cols_bytes() { return ((size_t)kNC * kLd + kNC + kN) * sizeof(double); }
 cudaError_t launch_bchain_cols(const HqChain* chains, int n, int dir, int b, cudaStream_t st) {
   k_bchain_cols<<<n * kCl, HQ_INT_THREADS, smem_bchain_cols_bytes(), st>>>(chains, n, dir, b);
   return cudaGetLastError();

@@ -60,6 +60,13 @@ k_measure(const HqChain* __restrict__ chains, int nchains, int dir, int b, int f
 //  CTA (blockIdx.y = 0: G(t,t), 1: G(t,0), 2: G(0,t)), except for the last slice which
 //  is rebuilt by the boundary step, and stores the per-slice results.
 // ---------------------------------------------------------------------------------
+template <bool RES>
+__device__ __forceinline__ void dyn_step(const HqChain& ch, double* M, int ld, int which, const double* vp, const double* vm,
+                                         double* stage) {
+  if (which != 2) apply_side<LEFT_B, RES, 1>(ch, M, ld, vp, stage);      // left multiplication by B(l) = e^V E
+  if (which != 1) apply_side<RIGHT_BINV, RES, 1>(ch, M, ld, vm, stage);  // right multiplication by B(l)^-1
+}
+
 __global__ void __launch_bounds__(HQ_INT_THREADS, 1)
 k_dyn_slices(const HqChain* __restrict__ chains, int nchains, int b, int flags, int resident) {
   extern __shared__ __align__(16) double smem[];
@@ -78,9 +85,11 @@ k_dyn_slices(const HqChain* __restrict__ chains, int nchains, int b, int flags, 
   double* M;
   int ld;
   double* p = smem;
-  if (resident) { M = p; ld = smem_ld(N); p += (size_t)N * ld; load_mat_async(M, ld, src, N, N); }
+  if (resident) { M = p; ld = interval_ld(N); p += (size_t)N * ld; load_mat_async(M, ld, src, N, N); }
   else { M = src; ld = N; }
   double* stage = p;
+  double* vp = stage + 8 * (pad16(N) + 4);
+  double* vm = vp + N;
   __syncthreads();
   const int nsl = t_hi - t_lo + 1;
   for (int step = 0; step < nsl; ++step) {
@@ -88,16 +97,10 @@ k_dyn_slices(const HqChain* __restrict__ chains, int nchains, int b, int flags, 
     const int l = t % ch.nt;
     for (int i = threadIdx.x; i < N; i += blockDim.x) s[i] = ch.fields[(size_t)l * N + i];
     __syncthreads();
-    if (which != 2) {  // left multiplication by B(l) = e^V E
-      apply_expk(ch, M, ld, 0, false, stage);
-      scale_rows(M, ld, N, s, ch.ev_p, ch.ev_m);
-      __syncthreads();
-    }
-    if (which != 1) {  // right multiplication by B(l)^-1 = E^-1 e^-V
-      apply_expk(ch, M, ld, 1, true, stage);
-      scale_cols(M, ld, N, s, ch.ev_m, ch.ev_p);
-      __syncthreads();
-    }
+    slice_factors(ch, s, vp, vm);
+    __syncthreads();
+    if (resident) dyn_step<true>(ch, M, ld, which, vp, vm, stage);
+    else dyn_step<false>(ch, M, ld, which, vp, vm, stage);
     if (step < nsl - 1 && snap) copy_mat(snap + (size_t)l * N * N, N, M, ld, N);
     __syncthreads();
   }
@@ -273,9 +276,11 @@ k_adj_interval(const HqChain* __restrict__ chains, int nchains, int b, int resid
   double* G;
   int ld;
   double* p = smem;
-  if (resident) { G = p; ld = smem_ld(N); p += (size_t)N * ld; load_mat_async(G, ld, ch.G, N, N); }
+  if (resident) { G = p; ld = interval_ld(N); p += (size_t)N * ld; load_mat_async(G, ld, ch.G, N, N); }
   else { G = ch.G; ld = N; }
   double* stage = p;
+  double* vp = stage + 8 * (pad16(N) + 4);
+  double* vm = vp + N;
   __syncthreads();
   const int nsl = t_hi - t_lo + 1;
   for (int step = 0; step < nsl; ++step) {
@@ -283,7 +288,10 @@ k_adj_interval(const HqChain* __restrict__ chains, int nchains, int b, int resid
     const int l = t % ch.nt;
     for (int i = threadIdx.x; i < N; i += blockDim.x) s[i] = ch.fields[(size_t)l * N + i];
     __syncthreads();
-    wrap_slice(ch, G, ld, s, HQ_UP, stage);
+    slice_factors(ch, s, vp, vm);
+    __syncthreads();
+    if (resident) wrap_slice<true>(ch, G, ld, vp, vm, HQ_UP, stage);
+    else wrap_slice<false>(ch, G, ld, vp, vm, HQ_UP, stage);
     if (step < nsl - 1) adj_accum(ch, G, ld, s, red);
     __syncthreads();
   }
@@ -327,6 +335,15 @@ size_t smem_udt_bytes(int Nmax, bool resident) {
 size_t smem_invert_bytes(int Nmax, bool resident) {
   return smem_matrix_bytes(Nmax, resident, 2 * kGJ * panel_ld(Nmax) + 3 * Nmax + 64);
 }
+// a matrix in the padded layout of the wrap, the stage of the dense exp(-dt K) and two words per site
+static size_t smem_wrap_bytes(int Nmax, bool resident) {
+  const size_t mat = resident ? (size_t)Nmax * interval_ld(Nmax) : 0;
+  return (mat + 8 * (pad16(Nmax) + 4) + 2 * (size_t)Nmax + 64) * sizeof(double);
+}
+// the B chain's matrix, the stage and one word per site
+static size_t smem_bchain_bytes(int Nmax, bool resident) {
+  return smem_matrix_bytes(Nmax, resident, 8 * (pad16(Nmax) + 4) + Nmax + 64);
+}
 size_t smem_matrix_bytes(int Nmax, bool resident, int extra_doubles) {
   const size_t mat = resident ? (size_t)Nmax * smem_ld(Nmax) : 0;
   return (mat + (size_t)extra_doubles) * sizeof(double);
@@ -365,23 +382,22 @@ bool interval_fits(int Nmax, int kmax, bool resident, size_t optin) {
 }
 
 bool matrices_fit(int Nmax, size_t optin) {
-  const size_t mat_stage = smem_matrix_bytes(Nmax, true, 8 * (((Nmax + 15) & ~15) + 4) + 64);
-  return interval_fits(Nmax, 4, true, optin) && mat_stage <= smem_room((const void*)k_bchain, optin) &&
-         mat_stage <= smem_room((const void*)k_dyn_slices, optin) &&
-         mat_stage <= smem_room((const void*)k_adj_interval, optin) &&
+  const size_t wrap = smem_wrap_bytes(Nmax, true);
+  return interval_fits(Nmax, 4, true, optin) && smem_bchain_bytes(Nmax, true) <= smem_room((const void*)k_bchain, optin) &&
+         wrap <= smem_room((const void*)k_dyn_slices, optin) && wrap <= smem_room((const void*)k_adj_interval, optin) &&
          smem_invert_bytes(Nmax, true) <= smem_room(fn_invert(), optin) &&
          smem_udt_bytes(Nmax, true) <= smem_room(fn_udt(), optin);
 }
 
 cudaError_t prepare_kernels(int Nmax, int kmax, bool resident) {
-  const size_t mat_stage = smem_matrix_bytes(Nmax, resident, 8 * (((Nmax + 15) & ~15) + 4) + 64);
+  const size_t wrap = smem_wrap_bytes(Nmax, resident);
   cudaError_t e;
   if ((e = raise_smem(0, fn_interval(), smem_interval_bytes(Nmax, kmax, resident))) != cudaSuccess) return e;
-  if ((e = raise_smem(1, (const void*)k_bchain, mat_stage)) != cudaSuccess) return e;
+  if ((e = raise_smem(1, (const void*)k_bchain, smem_bchain_bytes(Nmax, resident))) != cudaSuccess) return e;
   if ((e = raise_smem(2, fn_udt(), smem_udt_bytes(Nmax, resident))) != cudaSuccess) return e;
   if ((e = raise_smem(3, fn_invert(), smem_invert_bytes(Nmax, resident))) != cudaSuccess) return e;
-  if ((e = raise_smem(4, (const void*)k_dyn_slices, mat_stage)) != cudaSuccess) return e;
-  if ((e = raise_smem(5, (const void*)k_adj_interval, mat_stage)) != cudaSuccess) return e;
+  if ((e = raise_smem(4, (const void*)k_dyn_slices, wrap)) != cudaSuccess) return e;
+  if ((e = raise_smem(5, (const void*)k_adj_interval, wrap)) != cudaSuccess) return e;
   return cudaSuccess;
 }
 
@@ -392,7 +408,7 @@ cudaError_t prepare_interval_cl() {
 }
 
 cudaError_t launch_bchain(const HqChain* chains, int n, int dir, int b, int Nmax, bool resident, cudaStream_t st) {
-  const size_t bytes = smem_matrix_bytes(Nmax, resident, 8 * (((Nmax + 15) & ~15) + 4) + 64);
+  const size_t bytes = smem_bchain_bytes(Nmax, resident);
   k_bchain<<<n, HQ_INT_THREADS, bytes, st>>>(chains, n, dir, b, resident ? 1 : 0);
   return cudaGetLastError();
 }
@@ -405,7 +421,7 @@ cudaError_t launch_dyn_start(const HqChain* chains, int n, cudaStream_t st) {
   return cudaGetLastError();
 }
 cudaError_t launch_dyn_slices(const HqChain* chains, int n, int b, int flags, int Nmax, bool resident, cudaStream_t st) {
-  const size_t bytes = smem_matrix_bytes(Nmax, resident, 8 * (((Nmax + 15) & ~15) + 4) + 64);
+  const size_t bytes = smem_wrap_bytes(Nmax, resident);
   dim3 grid(n, 3);
   k_dyn_slices<<<grid, HQ_INT_THREADS, bytes, st>>>(chains, n, b, flags, resident ? 1 : 0);
   return cudaGetLastError();
@@ -419,7 +435,7 @@ cudaError_t launch_dyn_store(const HqChain* chains, int n, int b, cudaStream_t s
   return cudaGetLastError();
 }
 cudaError_t launch_adj_interval(const HqChain* chains, int n, int b, int Nmax, bool resident, cudaStream_t st) {
-  const size_t bytes = smem_matrix_bytes(Nmax, resident, 8 * (((Nmax + 15) & ~15) + 4) + 64);
+  const size_t bytes = smem_wrap_bytes(Nmax, resident);
   k_adj_interval<<<n, HQ_INT_THREADS, bytes, st>>>(chains, n, b, resident ? 1 : 0);
   return cudaGetLastError();
 }

@@ -1,7 +1,7 @@
 // hq_metropolis.cuh -- building blocks of the submatrix Metropolis update shared by the
 // interval kernels (one CTA per chain, and the thread-block-cluster variant for chains whose G
-// spans several SMs): the acceptance test, the warp walks of a site block, the panel
-// recurrences and the DMMA flush.
+// spans several SMs): the acceptance test, the warp walk of a site block, the panels of its
+// accepted flips and the DMMA flush.
 #pragma once
 #include "hq_common.cuh"
 
@@ -12,35 +12,43 @@ namespace hq {
 //
 //  The reference visits i = 0..N-1 in order, draws one uniform per site, and on
 //  acceptance applies G -= gamma G[:,i] (e_i^T - G[i,:]), gamma = Delta/(1+(1-G_ii)Delta)
-//  (src/hubbard.cpp:123-139). Here the sites are taken in blocks J of NB consecutive
+//  (src/hubbard.cpp:123-139). Here the sites are taken in blocks of up to 16 consecutive
 //  sites (E. Gull, P. Staar, S. Fuchs et al., Submatrix updates for the continuous-time
 //  auxiliary-field algorithm, Phys. Rev. B 83, 075122 (2011), applied to the Ising HS
 //  field):
-//   1. the walk: one warp holds g = G[J, J] in registers and visits the NB sites in order
+//   1. the walk: one warp holds g = G[B, B] in registers and visits the block's sites in order
 //      with the reference's acceptance test and rank-1 updates of g alone (every later
 //      decision of the block reads only g's diagonal). For the a accepted flips
-//      j_0 < j_1 < ... it records gamma_m, X[J, m] = gamma_m g[:, j_m] and
-//      Y[m, J] = g[j_m, :] - e_{j_m}^T (g before flip m);
+//      j_0 < j_1 < ... it records gamma_m, X[B, m] = gamma_m g[:, j_m] and
+//      Y[m, B] = g[j_m, :] - e_{j_m}^T (g before flip m);
 //   2. the a flips become the panels of G_new = G + X Y,
 //        X[:, m] = gamma_m (G[:, j_m] + sum_{m'<m} X[:, m'] Y[m', j_m])
 //        Y[m, :] = G[j_m, :] - e_{j_m}^T + sum_{m'<m} X[j_m, m'] Y[m', :]
-//      one row of X and one column of Y per thread, with the coefficients X[J, :] and
-//      Y[:, J] from the walk's records;
-//   3. G += X Y by DMMA (rank a <= NB) over all warps.
+//      one row of X and one column of Y per thread, with the coefficients X[B, :] and
+//      Y[:, B] from the walk's records;
+//   3. G += X Y by DMMA (rank a <= 16) over all warps.
+//  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 40, 18, 46;
+//  56, 28 and 85 with predicated record stores and a reciprocal with range checks in the walk, a
+//  branch per flip in the panels, and a flush that checked every element against the edge. The
+//  walk and the panels are bound by the latency of one dependency chain, the flush by the DMMA pipe.
+// ---------------------------------------------------------------------------------
+constexpr int kLdR = 18;  // leading dimension of the walk's records: 16-byte rows whose stores spread over the banks
+
 struct MetroShared {
   double* dl;     // Delta of each site [N]
+  double* thr;    // u (1 + Delta) of each site [N]
   double* u;      // uniforms [N]
   double* rr;     // visit-time ratio of each site [N] (ratio log)
   int8_t* s;      // fields of the slice [N]
   int8_t* flip;   // accepted flags [N]
-  double* X;      // N x 16 panel (column-major, ld panel_ld(N))
-  double* Y;      // 16 x N panel (row-major, ld panel_ld(N))
-  double* xt;     // X[J_s, m] of the block at xt[s * NB + m] (16-byte aligned)
-  double* yt;     // Y[m, J_s] of the block at yt[s * NB + m] (16-byte aligned)
-  int* ired;      // >= 8 ints
+  double* X;      // N x 16 panel (column-major)
+  double* Y;      // 16 x N panel (row-major)
+  double* xt;     // X[B_s, m] of the block at xt[s kLdR + m], for sites visited after flip m (16-byte aligned)
+  double* yt;     // Y[m, B_s] of the block at yt[s kLdR + m], likewise
+  double* qg;     // gamma of each panel column [16], then 16 words that idle lanes of the walk write to
+  int* ired;      // >= 2 ints: accepted counts of alternate blocks
   uint32_t* pw;   // a^(2i+1) mod m of each site [N]: the jump-ahead to site i's first draw
-  int* qj;        // accepted site of each panel column [16]
-  double* qg;     // gamma of each panel column [16]
+  int* qj;        // position inside the block of each accepted site, in order [16] (16-byte aligned)
 };
 
 // The acceptance ratio exactly as the reference evaluates it (src/hubbard.cpp:123-130):
@@ -51,125 +59,37 @@ __device__ __forceinline__ double reference_ratio(double gii, double dl) {
   return __ddiv_rn(__dmul_rn(a, a), __dadd_rn(1.0, dl));
 }
 
-// The Metropolis decision of src/dqmc_core.cpp:110: accept iff u < min(1, |r|). The fast walk
-// tests u (1 + Delta) < a^2 (thr = u (1 + Delta), 1 + Delta > 0), which needs no division on
-// its dependency chain and equals the reference's test except when the two sides lie within
-// a few rounding errors of each other. It only records whether that happened (thr and a are
-// the same in every lane, so the flag is warp-uniform; it is set with probability ~1e-12 per
-// proposal); the block is then walked again from its unchanged G with the reference's own
-// form, u < min(1, |r|) with r as the reference evaluates it, for every decision.
-template <bool EXACT>
-__device__ __forceinline__ bool accept_flip(double thr, double av, double gii, double dl, const double* u, bool& near) {
-  if (EXACT) return *u < fmin(1.0, fabs(reference_ratio(gii, dl)));
-  const double a2 = av * av;
-  near = near || fabs(thr - a2) <= 1e-12 * a2;
-  return thr < a2;
+// 1 / x, correctly rounded for the walk's arguments (normal numbers): the hardware's approximation
+// (relative error below 2^-23) and two Newton steps y + y (1 - x y), whose FMA residuals leave 2^-92
+// before the last rounding. Without the range checks and the branch of the intrinsic, whose value
+// it has, the sites of a block are one stretch of straight code.
+__device__ __forceinline__ double reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 
-// the walk of the block [b0, b0 + nb) by one warp (see above); writes the records and the
-// accepted count into ired[slot]; returns the near-tie flag of the fast walk. LOGT false
-// compiles the ratio log out (log is then ignored).
-template <int NB, bool EXACT, bool LOGT = true>
-__device__ __forceinline__ bool walk_block(const HqChain& ch, const double* G, int ld, const MetroShared& sh, int b0, int nb,
-                           bool log, int slot) {
-  log = LOGT && log;
-  constexpr int R = (NB * NB >= 32) ? NB * NB / 32 : 1;  // rows of g held by one lane
-  constexpr int H = NB / R;                              // lane groups (rows h*R .. h*R+R-1)
-  const int lane = threadIdx.x & 31;
-  // lane layout of g: lane le = h * NB + c holds g[h*R + i][c], i < R (lanes >= NB*H mirror)
-  const int le = lane % (NB * H), c = le % NB, h = le / NB;
-  const bool writer = lane < NB * H;
-  double r[R];
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int row = h * R + i;
-    r[i] = (row < nb && c < nb) ? G[b0 + row + (size_t)(b0 + c) * ld] : 0.0;
-  }
-  // per-site constants of the block, loaded before the walk (the walk's shared-memory
-  // stores would otherwise order every later load behind them)
-  double dls[NB], thr[NB];
-#pragma unroll
-  for (int s = 0; s < NB; ++s) {
-    dls[s] = s < nb ? sh.dl[b0 + s] : 0.0;
-    thr[s] = s < nb ? sh.u[b0 + s] * (1.0 + dls[s]) : 0.0;
-  }
-  // per-site records stay in registers during the walk (shared-memory stores would queue
-  // with the shuffles on the same pipe): xk[s] = X[J_row, s] for the row this lane writes,
-  // yk[s] = Y[s, J_c], the acceptance mask and, in lane s, gamma_s and the visit ratio
-  double xk[NB], yk[NB], myg = 0.0, myr = 0.0;
-  unsigned mask = 0u;
-  bool near = false;  // a decision came within rounding of the other side (fast walk only)
-#pragma unroll
-  for (int s = 0; s < NB; ++s) {
-    xk[s] = 0.0;
-    yk[s] = 0.0;
-    if (s < nb) {
-      const int ss = s / R, si = s % R;  // g[s][*] is held by group ss at register si
-      // column s, row s and the diagonal entry of the current g. On the step's dependency
-      // chain (g_ss -> a -> 1/a -> the rank-1 update -> the next g_ss): a as one FMA on
-      // 1 + Delta, the correctly rounded reciprocal of a (formed before the decision so that
-      // it overlaps the test), and one product with the column, which was scaled by Delta
-      // beside the chain
-      const double dg = __shfl_sync(0xffffffffu, r[si], ss * NB + s);
-      double colr[R];
-#pragma unroll
-      for (int i = 0; i < R; ++i) colr[i] = __shfl_sync(0xffffffffu, r[i], h * NB + s);
-      const double yv = __shfl_sync(0xffffffffu, r[si], ss * NB + c) - (c == s ? 1.0 : 0.0);
-      const double dl = dls[s];
-      const double av = fma(-dg, dl, 1.0 + dl);  // 1 + (1 - g_ss) Delta
-      const double rc = __drcp_rn(av);
-      const double gam = dl * rc;                // Delta / a
-      if (LOGT && log && lane == s) myr = reference_ratio(dg, dl);
-      // accept iff u < min(1, |r|), r = a^2 / (1 + Delta), 1 + Delta = e^{-2 alpha s} > 0
-      const bool acc = accept_flip<EXACT>(thr[s], av, dg, dl, sh.u + b0 + s, near);
-      const double ge = acc ? gam : 0.0;
-      const double gr = acc ? rc : 0.0;
-      double xs = colr[0];
-#pragma unroll
-      for (int i = 1; i < R; ++i) xs = (c == i) ? colr[i] : xs;
-      xk[s] = ge * xs;
-      yk[s] = yv;
-      if (lane == s) myg = gam;
-#pragma unroll
-      for (int i = 0; i < R; ++i) r[i] = fma(gr * (dl * colr[i]), yv, r[i]);
-      mask |= acc ? (1u << s) : 0u;
-    }
-  }
-  // the records of the accepted flips, in acceptance order
-  const int a = __popc(mask);
-#pragma unroll
-  for (int s = 0; s < NB; ++s) {
-    if (mask & (1u << s)) {
-      const int m = __popc(mask & ((1u << s) - 1u));
-      if (writer && c < R) sh.xt[(h * R + c) * NB + m] = xk[s];
-      if (writer && h == 0) sh.yt[c * NB + m] = yk[s];
-    }
-  }
-  if (lane < nb) {
-    const bool acc = (mask >> lane) & 1u;
-    if (acc) {
-      const int m = __popc(mask & ((1u << lane) - 1u));
-      sh.qj[m] = b0 + lane;
-      sh.qg[m] = myg;
-    }
-    sh.flip[b0 + lane] = acc ? 1 : 0;
-    if (log) sh.rr[b0 + lane] = myr;
-  }
-  if (lane == 0) sh.ired[slot] = a;
-  return near;
-}
-
-// the walk of a 16-site block with g tiled 4 rows x 2 columns per lane: lane 8 rg + cg holds
-// g[4 rg + a][2 cg + b] (a < 4, b < 2). A step needs column s for the lane's four rows, row s
-// for its two columns and the diagonal entry: 7 shuffles instead of the 10 of an 8 x 1 tile.
-// Every entry is updated with the same expression as in walk_block, so the two walks agree
-// bitwise. Records: lanes with cg < 4 write X[J_(4 rg + cg), m], lanes with rg < 2 write
-// Y[m, J_(2 cg + rg)].
-template <bool EXACT, bool LOGT = true>
-__device__ __forceinline__ bool walk_block16(const HqChain& ch, const double* G, int ld, const MetroShared& sh, int b0,
-                                             int nb, bool log, int slot) {
+// The walk of the nb <= 16 sites [b0, b0 + nb) by one warp. Lane 8 rg + cg holds the entries
+// (4 rg + a, 2 cg + b), a < 4, b < 2, of g: a step needs column s at the lane's four rows, row s at its
+// two columns and the diagonal entry, 7 shuffles. Entries of rows and columns already visited are
+// not read again; they are left to run along.
+//
+// The decision of src/dqmc_core.cpp:110 is accept iff u < min(1, |r|). The fast walk tests
+// u (1 + Delta) < a^2 (1 + Delta > 0), which needs no division on its dependency chain and equals
+// the reference's test except when the two sides lie within a few rounding errors of each other.
+// It only records whether that happened (warp-uniform; probability ~1e-12 per proposal): the
+// return value. The caller then walks the block again, from its unchanged G, with EXACT: every
+// decision in the reference's own form, u < min(1, |r|) with r as the reference evaluates it.
+// The one warp issues in order, so the walk is straight code: every lane stores its records (lanes
+// without any to a spare word), of accepted sites and others alike (the next site's overwrite them),
+// because predicated stores became branches with a reconvergence each (5.5k instead of 3.2k cycles
+// per block); the sites' constants are in registers before the first store (3.2k -> 2.9k); and
+// NBC = 16 fixes nb at compile time (NBC = 0 takes nb). LOGT false compiles the ratio log out.
+template <bool EXACT, bool LOGT, int NBC>
+__device__ __forceinline__ bool walk_block16(const double* G, int ld, const MetroShared& sh, int b0, int nbr, int slot) {
   constexpr int NB = 16;
-  log = LOGT && log;
+  const int nb = NBC > 0 ? NBC : nbr;
   const int lane = threadIdx.x & 31;
   const int rg = lane >> 3, cg = lane & 7;
   double r[4][2];
@@ -180,127 +100,189 @@ __device__ __forceinline__ bool walk_block16(const HqChain& ch, const double* G,
       const int row = 4 * rg + a, col = 2 * cg + b;
       r[a][b] = (row < nb && col < nb) ? G[b0 + row + (size_t)(b0 + col) * ld] : 0.0;
     }
-  double dls[NB], thr[NB];
+  double dls[NB], thrs[NB];
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
     dls[s] = s < nb ? sh.dl[b0 + s] : 0.0;
-    thr[s] = s < nb ? sh.u[b0 + s] * (1.0 + dls[s]) : 0.0;
+    thrs[s] = s < nb ? sh.thr[b0 + s] : 0.0;
   }
-  double xk[NB], yk[NB], myg = 0.0, myr = 0.0;
+  // this lane's record row is 4 rg + cg (cg < 4), its record column 2 cg + rg (rg < 2)
+  double* xrec = cg < 4 ? sh.xt + (4 * rg + cg) * kLdR : sh.qg + 16;
+  double* yrec = rg < 2 ? sh.yt + (2 * cg + rg) * kLdR : sh.qg + 16;
+  double myr = 0.0;
   unsigned mask = 0u;
-  bool near = false;  // a decision came within rounding of the other side (fast walk only)
+  bool near = false;
+  int m = 0;  // flips accepted so far
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
-    xk[s] = 0.0;
-    yk[s] = 0.0;
     if (s < nb) {
-      // g[s][s]; column s at the lane's rows (held by lane 8 rg + s/2, column slot s&1);
-      // row s at the lane's columns (held by lane 8 (s/4) + cg, row slot s&3)
+      const double dl = dls[s], thr = thrs[s];
+      // g_ss (lane 8 (s/4) + s/2); column s at the lane's rows (lane 8 rg + s/2, slot s&1); row s at
+      // the lane's columns (lane 8 (s/4) + cg, slot s&3)
       const double dg = __shfl_sync(0xffffffffu, r[s & 3][s & 1], 8 * (s >> 2) + (s >> 1));
-      double colr[4];
+      double col[4], row[2];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) colr[a] = __shfl_sync(0xffffffffu, r[a][s & 1], 8 * rg + (s >> 1));
-      double rowv[2];
+      for (int a = 0; a < 4; ++a) col[a] = __shfl_sync(0xffffffffu, r[a][s & 1], 8 * rg + (s >> 1));
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
-        rowv[b] = __shfl_sync(0xffffffffu, r[s & 3][b], 8 * (s >> 2) + cg) - (2 * cg + b == s ? 1.0 : 0.0);
-      const double dl = dls[s];
-      const double av = fma(-dg, dl, 1.0 + dl);  // 1 + (1 - g_ss) Delta (as in walk_block)
-      const double rc = __drcp_rn(av);
-      const double gam = dl * rc;                // Delta / a
-      if (LOGT && log && lane == s) myr = reference_ratio(dg, dl);
-      const bool acc = accept_flip<EXACT>(thr[s], av, dg, dl, sh.u + b0 + s, near);
-      const double ge = acc ? gam : 0.0;
+      for (int b = 0; b < 2; ++b) row[b] = __shfl_sync(0xffffffffu, r[s & 3][b], 8 * (s >> 2) + cg);
+      const double av = fma(-dg, dl, 1.0 + dl);  // 1 + (1 - g_ss) Delta
+      const double rc = reciprocal(av);
+      const double gam = dl * rc;                // gamma = Delta / av
+      if (LOGT && lane == s) myr = reference_ratio(dg, dl);
+      bool acc;
+      if (EXACT) {
+        acc = sh.u[b0 + s] < fmin(1.0, fabs(reference_ratio(dg, dl)));
+      } else {
+        const double a2 = av * av;
+        near = near || fabs(thr - a2) <= 1e-12 * a2;
+        acc = thr < a2;
+      }
+      // the records of the flip, read for sites visited later
+      const double xs = (cg & 1) ? ((cg & 2) ? col[3] : col[1]) : ((cg & 2) ? col[2] : col[0]);
+      xrec[m] = gam * xs;
+      yrec[m] = (rg & 1) ? row[1] : row[0];
+      sh.qj[m] = s;
+      sh.qg[m] = gam;
       const double gr = acc ? rc : 0.0;
-      // the record row of this lane is 4 rg + cg (cg < 4), its record column 2 cg + rg (rg < 2)
-      double xs = colr[0];
-      xs = (cg == 1) ? colr[1] : xs;
-      xs = (cg == 2) ? colr[2] : xs;
-      xs = (cg == 3) ? colr[3] : xs;
-      xk[s] = ge * xs;
-      yk[s] = (rg & 1) ? rowv[1] : rowv[0];
-      if (lane == s) myg = gam;
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
-        const double f = gr * (dl * colr[a]);
+        const double f = gr * (dl * col[a]);
 #pragma unroll
-        for (int b = 0; b < 2; ++b) r[a][b] = fma(f, rowv[b], r[a][b]);
+        for (int b = 0; b < 2; ++b) r[a][b] = fma(f, row[b], r[a][b]);
       }
       mask |= acc ? (1u << s) : 0u;
+      m += acc ? 1 : 0;
     }
   }
-  const int a = __popc(mask);
-#pragma unroll
-  for (int s = 0; s < NB; ++s) {
-    if (mask & (1u << s)) {
-      const int m = __popc(mask & ((1u << s) - 1u));
-      if (cg < 4) sh.xt[(4 * rg + cg) * NB + m] = xk[s];
-      if (rg < 2) sh.yt[(2 * cg + rg) * NB + m] = yk[s];
-    }
-  }
+  if (!EXACT && near) return true;
   if (lane < nb) {
-    const bool acc = (mask >> lane) & 1u;
-    if (acc) {
-      const int m = __popc(mask & ((1u << lane) - 1u));
-      sh.qj[m] = b0 + lane;
-      sh.qg[m] = myg;
-    }
-    sh.flip[b0 + lane] = acc ? 1 : 0;
-    if (log) sh.rr[b0 + lane] = myr;
+    sh.flip[b0 + lane] = (mask >> lane) & 1u;
+    if (LOGT) sh.rr[b0 + lane] = myr;
   }
-  if (lane == 0) sh.ired[slot] = a;
-  return near;
+  if (lane == 0) sh.ired[slot] = m;
+  return false;
 }
 
-// panels of the a flips of block [b0, b0 + NB): the two triangular recurrences, one row of X
-// and one column of Y per thread; the coefficients of flip m are contiguous in the records
-// (xt / yt at row j_m - b0) and are read in 16-byte pairs
-template <int NB>
+// the walks of the ratio log, of near ties and of short blocks, out of line: their code and
+// registers do not weigh on the fast walk's
+template <bool EXACT, bool LOGT>
+__device__ __noinline__ bool walk_rare(const double* G, int ld, const MetroShared sh, int b0, int nb, int slot) {
+  return walk_block16<EXACT, LOGT, 0>(G, ld, sh, b0, nb, slot);
+}
+// the walk with the reference's form of every decision where the fast one came near a tie
+__device__ __forceinline__ void walk(const double* G, int ld, const MetroShared& sh, int b0, int nb, bool log, int slot) {
+  if (log) {
+    if (walk_rare<false, true>(G, ld, sh, b0, nb, slot)) walk_rare<true, true>(G, ld, sh, b0, nb, slot);
+  } else if (nb == 16) {
+    if (walk_block16<false, false, 16>(G, ld, sh, b0, nb, slot)) walk_rare<true, false>(G, ld, sh, b0, nb, slot);
+  } else {
+    if (walk_rare<false, false>(G, ld, sh, b0, nb, slot)) walk_rare<true, false>(G, ld, sh, b0, nb, slot);
+  }
+}
+
+// W lines of a panel for a flips, 4 (KA - 1) < a <= 4 KA, in the thread's registers,
+//   v[m] = w_m (g[m] + sum_{m'<m} c[j_m][m'] v[m']):
+// rows of X (ISX: g[m] = G[p, j_m], c = the records yt, w = gamma) or columns of Y (g[m] = G[j_m, p] less
+// 1 where p = j_m, c = xt, w = 1); entry of flip m at g[w] + q_m gs, delta[w] the position q_m of the 1.
+// The sums run over the even and the odd m' apart. There is no branch on a (flips past a come out
+// as zero), so the loads run ahead of the recurrences; two lines per thread share the coefficients,
+// whose broadcast loads are most of the shared-memory traffic.
+template <int KA, int W, bool ISX>
+__device__ __forceinline__ void panel_lines(const double* const (&g)[W], size_t gs, const int (&delta)[W], const MetroShared& sh,
+                                            int a, double (&v)[W][4 * KA]) {
+  constexpr int K = 4 * KA;
+  int qm[K];
+#pragma unroll
+  for (int k = 0; k < KA; ++k) {
+    const int4 t = *reinterpret_cast<const int4*>(sh.qj + 4 * k);
+    qm[4 * k] = t.x; qm[4 * k + 1] = t.y; qm[4 * k + 2] = t.z; qm[4 * k + 3] = t.w;
+  }
+#pragma unroll
+  for (int m = 0; m < K; ++m) {
+    qm[m] = m < a ? qm[m] : 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      v[w][m] = g[w][qm[m] * gs];
+      if (!ISX) v[w][m] -= (qm[m] == delta[w] ? 1.0 : 0.0);
+    }
+  }
+  const double* rec = ISX ? sh.yt : sh.xt;
+#pragma unroll
+  for (int m = 0; m < K; ++m) {
+    const double* c = rec + qm[m] * kLdR;
+    double s0[W], s1[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      s0[w] = v[w][m];
+      s1[w] = 0.0;
+    }
+#pragma unroll
+    for (int m2 = 0; m2 + 1 < m; m2 += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(c + m2);
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        s0[w] = fma(v[w][m2], t.x, s0[w]);
+        s1[w] = fma(v[w][m2 + 1], t.y, s1[w]);
+      }
+    }
+    const double cl = (m & 1) ? c[m - 1] : 0.0;
+    const double sc = ISX ? sh.qg[m] : 1.0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      if (m & 1) s0[w] = fma(v[w][m - 1], cl, s0[w]);
+      const double t = ISX ? sc * (s0[w] + s1[w]) : s0[w] + s1[w];
+      v[w][m] = m < a ? t : 0.0;
+    }
+  }
+}
+// rows t and t + ceil(N / 2) of X (t + ... past the last row repeats it) by threads 0 .. 127
+template <int KA>
+__device__ __forceinline__ void panel_rows(const double* Gb, int ld, int N, const MetroShared& sh, int a, int ldx) {
+  const int H = (N + 1) / 2;
+  for (int t = threadIdx.x & 127; t < H; t += 128) {
+    const int p1 = min(t + H, N - 1);
+    const double* g[2] = {Gb + t, Gb + p1};
+    const int none[2] = {-1, -1};
+    double v[2][4 * KA];
+    panel_lines<KA, 2, true>(g, ld, none, sh, a, v);
+#pragma unroll
+    for (int m = 0; m < 4 * KA; ++m) {
+      sh.X[t + m * ldx] = v[0][m];
+      sh.X[p1 + m * ldx] = v[1][m];
+    }
+  }
+}
+// columns t and t + ceil(nc / 2) of Y by threads 128 .. 255: Gr = the block's first row of the nc
+// columns, the first of them column c0 of G
+template <int KA>
+__device__ __forceinline__ void panel_cols(const double* Gr, int ld, int nc, int c0, const MetroShared& sh, int a, int b0,
+                                           int ldy) {
+  const int H = (nc + 1) / 2;
+  for (int t = threadIdx.x & 127; t < H; t += 128) {
+    const int p1 = min(t + H, nc - 1);
+    const double* g[2] = {Gr + (size_t)t * ld, Gr + (size_t)p1 * ld};
+    const int delta[2] = {c0 + t - b0, c0 + p1 - b0};
+    double v[2][4 * KA];
+    panel_lines<KA, 2, false>(g, 1, delta, sh, a, v);
+#pragma unroll
+    for (int m = 0; m < 4 * KA; ++m) {
+      sh.Y[m * ldy + t] = v[0][m];
+      sh.Y[m * ldy + p1] = v[1][m];
+    }
+  }
+}
+// both panels of the block at b0 on one CTA
+template <int KA>
 __device__ __forceinline__ void build_panels(const double* G, int ld, int N, const MetroShared& sh, int ldp, int a, int b0) {
-  for (int p = threadIdx.x; p < N; p += blockDim.x) {
-    double x[NB], y[NB];
-#pragma unroll
-    for (int m = 0; m < NB; ++m) {
-      x[m] = 0.0;
-      y[m] = 0.0;
-      if (m < a) {
-        const int jm = sh.qj[m], sj = jm - b0;
-        const double* cy = sh.yt + sj * NB;  // Y[m2, j_m]
-        const double* cx = sh.xt + sj * NB;  // X[j_m, m2]
-        double cx0 = G[p + (size_t)jm * ld], cx1 = 0.0;
-        double cy0 = G[jm + (size_t)p * ld] - (p == jm ? 1.0 : 0.0), cy1 = 0.0;
-#pragma unroll
-        for (int m2 = 0; m2 + 1 < m; m2 += 2) {
-          const double2 vy = *reinterpret_cast<const double2*>(cy + m2);
-          const double2 vx = *reinterpret_cast<const double2*>(cx + m2);
-          cx0 = fma(x[m2], vy.x, cx0);
-          cx1 = fma(x[m2 + 1], vy.y, cx1);
-          cy0 = fma(vx.x, y[m2], cy0);
-          cy1 = fma(vx.y, y[m2 + 1], cy1);
-        }
-        if (m & 1) {
-          cx0 = fma(x[m - 1], cy[m - 1], cx0);
-          cy0 = fma(cx[m - 1], y[m - 1], cy0);
-        }
-        x[m] = sh.qg[m] * (cx0 + cx1);
-        y[m] = cy0 + cy1;
-      }
-    }
-    // stores after the recurrence: the loads above are free to run ahead of them
-#pragma unroll
-    for (int m = 0; m < NB; ++m) {
-      if (m < a) {
-        sh.X[p + m * ldp] = x[m];
-        sh.Y[m * ldp + p] = y[m];
-      }
-    }
-  }
+  static_assert(HQ_INT_THREADS == 256, "half the threads take X, half Y");
+  if (threadIdx.x < 128) panel_rows<KA>(G + (size_t)b0 * ld, ld, N, sh, a, ldp);
+  else panel_cols<KA>(G + b0, ld, N, 0, sh, a, b0, ldp);
 }
 
-// G[0:M, 0:Nc] += X[:, 0:k] Y[0:k, :] (k <= 16): 48 x 32 warp tiles (3 x 4 DMMA tiles sharing
-// their fragments; 144 = 3 x 48), all warps
-__device__ __forceinline__ void rank_update48(double* G, int ld, int M, int Nc, const double* X, int ldx, const double* Y, int ldy,
-                              int k) {
+// G[0:M, 0:Nc] += X[:, 0:k] Y[0:k, :] (k <= 16) with every element
+// checked against the edge: 48 x 32 warp tiles (3 x 4 DMMA tiles sharing their fragments). For G in
+// global memory, whose columns are not padded.
+__device__ __forceinline__ void rank_update48(double* G, int ld, int M, int Nc, const MetroShared& sh, int ldx, int ldy, int k) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, q = lane & 3;
   const int mt = (M + 47) / 48, ns = (Nc + 31) / 32;
@@ -323,17 +305,18 @@ __device__ __forceinline__ void rank_update48(double* G, int ld, int M, int Nc, 
       if (s < ksteps) {
         const int m = 4 * s + q;
         const bool mk = m < k;
+        const double* Xp = sh.X + m * ldx;
         double fa[3][2], fb[4];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           const int r = r0 + 16 * i + g;
-          fa[i][0] = (r < M && mk) ? X[r + m * ldx] : 0.0;
-          fa[i][1] = (r + 8 < M && mk) ? X[r + 8 + m * ldx] : 0.0;
+          fa[i][0] = (r < M && mk) ? Xp[r] : 0.0;
+          fa[i][1] = (r + 8 < M && mk) ? Xp[r + 8] : 0.0;
         }
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const int cb = c0 + t * 8 + g;
-          fb[t] = (cb < Nc && mk) ? Y[m * ldy + cb] : 0.0;
+          fb[t] = (cb < Nc && mk) ? sh.Y[m * ldy + cb] : 0.0;
         }
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -354,9 +337,58 @@ __device__ __forceinline__ void rank_update48(double* G, int ld, int M, int Nc, 
   }
 }
 
-// the flush of one block's flips, G[0:N, 0:N] += X[:, 0:k] Y[0:k, :]
-__device__ __forceinline__ void flush_block(double* G, int ld, int N, const double* X, int ldx, const double* Y, int ldy, int k) {
-  rank_update48(G, ld, N, N, X, ldx, Y, ldy, k);
+// G[0:16 MT, 0:8 T] += X[:, 0:4 KS] Y[0:4 KS, :] on storage that is padded to whole DMMA tiles, so that
+// nothing is checked: 16 x 8 NT strips, NT = 3 or 2, whichever divides T (tile_cols). Pad rows and
+// columns hold any values; they only reach pad rows and columns.
+// Bound by the DMMA pipe (12 x 12, rank 12: 162 tiles x 3 steps x 8 cycles = 3.9k of 5.2k
+// measured); strips of 16 x 24 keep eight warps evenly loaded (54 strips), 48 x 32 tiles took 7.1k.
+template <int MT, int T, int KS>
+__device__ __forceinline__ void rank_strips(double* G, int ld, const MetroShared& sh, int ldx, int ldy) {
+  constexpr int NT = T % 3 == 0 ? 3 : 2;
+  constexpr int NG = T / NT;
+  static_assert(T % NT == 0, "tile_cols pads the columns to whole strips");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, q = lane & 3;
+  const double* Xq = sh.X + q * ldx + g;
+  const double* Yq = sh.Y + q * ldy + g;
+#pragma unroll 1
+  for (int st = warp; st < MT * NG; st += nw) {
+    const int r0 = (st % MT) * 16, t0 = (st / MT) * NT;
+    double* Gp = G + r0 + g + (size_t)(8 * t0 + 2 * q) * ld;
+    const double* Yp = Yq + 8 * t0;
+    double acc[NT][4];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      acc[t][0] = Gp[(8 * t) * ld];
+      acc[t][1] = Gp[(8 * t + 1) * ld];
+      acc[t][2] = Gp[8 + (8 * t) * ld];
+      acc[t][3] = Gp[8 + (8 * t + 1) * ld];
+    }
+#pragma unroll
+    for (int s = 0; s < KS; ++s) {
+      const double a0 = Xq[4 * s * ldx + r0], a1 = Xq[4 * s * ldx + r0 + 8];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) dmma_16x8x4(acc[t], a0, a1, Yp[4 * s * ldy + 8 * t]);
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      Gp[(8 * t) * ld] = acc[t][0];
+      Gp[(8 * t + 1) * ld] = acc[t][1];
+      Gp[8 + (8 * t) * ld] = acc[t][2];
+      Gp[8 + (8 * t + 1) * ld] = acc[t][3];
+    }
+  }
+}
+
+// calls f(integral constant ceil(a / 4)) for 1 <= a <= 16 flips
+template <class F>
+__device__ __forceinline__ void for_ksteps(int a, F&& f) {
+  switch ((a + 3) >> 2) {
+    case 1: f(IntC<1>{}); break;
+    case 2: f(IntC<2>{}); break;
+    case 3: f(IntC<3>{}); break;
+    default: f(IntC<4>{}); break;
+  }
 }
 
 }  // namespace hq

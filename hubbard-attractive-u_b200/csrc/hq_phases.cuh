@@ -16,7 +16,7 @@ namespace hq {
 //  direction without updates.
 // ---------------------------------------------------------------------------------
 // The B products of interval b applied to the top of the pushing stack (X = U_top D_top, or 1),
-// into ch.X. `smem` is the dynamic region (N x smem_ld(N) when resident, then the stage); s holds
+// into ch.X. `smem` is the dynamic region (N x smem_ld(N) when resident, then the stage and N words); s holds
 // N fields (shared). keep_x (resident only): X stays at the start of `smem` (leading dimension
 // smem_ld(N)) for the factorisation that follows in the same block, instead of going to ch.X.
 // Every thread of the block calls it; the chain is active and b < n_stab.
@@ -32,6 +32,7 @@ __device__ __forceinline__ void bchain_body(const HqChain& ch, int dir, int b, b
   double* p = smem;
   if (resident) { X = p; ld = smem_ld(N); p += (size_t)N * ld; } else { X = ch.X; ld = N; }
   double* stage = p;
+  double* v = stage + 8 * (pad16(N) + 4);  // e^{V} of a slice
   const size_t NN = (size_t)N * N;
   const double* U = top >= 0 ? ch.stackU + ((size_t)side * ch.n_stab + top) * NN : nullptr;
   const double* D = top >= 0 ? ch.stackD + ((size_t)side * ch.n_stab + top) * N : nullptr;
@@ -54,18 +55,15 @@ __device__ __forceinline__ void bchain_body(const HqChain& ch, int dir, int b, b
     const int l = t % ch.nt;
     for (int i = threadIdx.x; i < N; i += blockDim.x) s[i] = ch.fields[(size_t)l * N + i];
     __syncthreads();
-    if (ch.expk_mode == HQK_EXPK_SEPARABLE) {
-      // e^{V} rides on the first pass (down: before expK) or the last pass (up: after it)
-      if (dir == HQ_DOWN) sep_apply_any<1, 0>(X, ld, N, ch.L, ch.sep_a, ch.sep_c, 0, s, ch.ev_p, ch.ev_m, 1.0, 1.0);
-      else sep_apply_any<0, 2>(X, ld, N, ch.L, ch.sep_a, ch.sep_c, 0, s, ch.ev_p, ch.ev_m, 1.0, 1.0);
-    } else if (dir == HQ_DOWN) {
-      scale_rows(X, ld, N, s, ch.ev_p, ch.ev_m);
-      __syncthreads();
-      apply_expk(ch, X, ld, 0, false, stage);
+    // e^{V} rides on the first pass (down: before expK) or the last pass (up: after it)
+    slice_factors(ch, s, v, nullptr);
+    __syncthreads();
+    if (resident) {
+      if (dir == HQ_DOWN) apply_side<LEFT_BT, true, 0>(ch, X, ld, v, stage);
+      else apply_side<LEFT_B, true, 0>(ch, X, ld, v, stage);
     } else {
-      apply_expk(ch, X, ld, 0, false, stage);
-      scale_rows(X, ld, N, s, ch.ev_p, ch.ev_m);
-      __syncthreads();
+      if (dir == HQ_DOWN) apply_side<LEFT_BT, false, 0>(ch, X, ld, v, stage);
+      else apply_side<LEFT_B, false, 0>(ch, X, ld, v, stage);
     }
   }
   if (resident && !keep_x) copy_mat(ch.X, N, X, ld, N);

@@ -115,7 +115,7 @@ __device__ int2 take_item(const int2* __restrict__ cinfo, int nchains, int nitem
 
 // doubles of the B-chain region (matrix + stage), after which its fields of one slice sit
 __host__ __device__ inline size_t bchain_doubles(int N) {
-  return (size_t)N * smem_ld(N) + 8 * (((N + 15) & ~15) + 4) + 64;
+  return (size_t)N * smem_ld(N) + 8 * (pad16(N) + 4) + N + 64;
 }
 
 __global__ void __launch_bounds__(HQ_INT_THREADS, 1)
@@ -170,7 +170,7 @@ k_sweep(const HqChain* __restrict__ chains, int nchains, const int2* __restrict_
       const IntervalScratch sc = interval_scratch_at(smem + off);
       if (threadIdx.x == 0) mbar_init(sc.gbar, 1);
       __syncthreads();
-      interval_body(ch, dir, b, flags, true, smem, sc, 0u);
+      interval_body<true>(ch, dir, b, flags, smem, sc, 0u);
       // the bulk store of G has completed (warp 0 waited for it): order it before the generic
       // accesses of the phases below
       if (threadIdx.x < 32) fence_proxy_async_all();

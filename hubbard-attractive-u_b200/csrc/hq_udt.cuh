@@ -540,9 +540,9 @@ __device__ __forceinline__ void udt_body(const HqChain& ch, int side, int b, boo
     phase(5);
     for (int t = threadIdx.x; t < kQB * kQB; t += blockDim.x) {
       const int l = t / kQB, j = t % kQB;
+      if (j >= m) continue;  // W has leading dimension ldp, which N < 16 may leave below kQB
       double acc = 0.0;
-      if (j < m)
-        for (int l2 = 0; l2 < kQB; ++l2) acc = fma(Tp[l * kQB + l2], Vb[(p0 + j) + l2 * ldp], acc);
+      for (int l2 = 0; l2 < kQB; ++l2) acc = fma(Tp[l * kQB + l2], Vb[(p0 + j) + l2 * ldp], acc);
       W[l * ldp + j] = -acc;
     }
     for (int idx = threadIdx.x; idx < N * m; idx += blockDim.x) {
