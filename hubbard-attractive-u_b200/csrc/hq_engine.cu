@@ -135,12 +135,40 @@ void host_gemm(int n, const double* A, bool ta, const double* B, bool tb, double
     }
 }
 
+// Eigen-decomposition of K = -t H_nn - mu 1 on the L x L torus in closed form: the columns of Q are
+// the products of the real Fourier modes of the two directions, H_1d has the eigenvalues
+// 2 cos(2 pi k / L) (any orthonormal eigenbasis serves the adjoint alike).
+void lattice_eig(int L, double t, double mu, double* w, double* Q) {
+  const long double pi = 3.14159265358979323846264338327950288L;
+  std::vector<double> F(size_t(L) * L), lam(L);  // F[x + L a]: mode a at x
+  for (int a = 0; a < L; ++a) {
+    const int k = (a + 1) / 2;  // modes 0, 1c, 1s, 2c, 2s, ...
+    lam[a] = static_cast<double>(2.0L * std::cos(2.0L * pi * k / L));
+    for (int x = 0; x < L; ++x) {
+      const long double th = 2.0L * pi * ((long long)k * x % L) / L;
+      const bool alone = k == 0 || 2 * k == L;
+      const long double v = alone ? std::cos(th) / std::sqrt((long double)L)
+                                  : std::sqrt(2.0L / L) * (a % 2 ? std::cos(th) : std::sin(th));
+      F[x + size_t(L) * a] = static_cast<double>(v);
+    }
+  }
+  const int N = L * L;
+  for (int b = 0; b < L; ++b)
+    for (int a = 0; a < L; ++a) {
+      const int j = a + L * b;
+      w[j] = -t * (lam[a] + lam[b]) - mu;
+      for (int y = 0; y < L; ++y)
+        for (int x = 0; x < L; ++x) Q[(x + L * y) + size_t(j) * N] = F[x + size_t(L) * a] * F[y + size_t(L) * b];
+    }
+}
+
 struct ChainHost {
   hq_chain_params p;
   int N, n_stab, kmax, expk_mode;
   bool custom_hop = false;
   std::vector<double> hop;     // N x N hopping (custom or nearest neighbour)
   std::vector<double> K;       // N x N
+  std::vector<double> eig_w, eig_Q;  // eigen-decomposition of a custom K (hq_set_hopping)
   double alpha, dt;
   uint32_t rng_after_fields = 0;
   bool fields_set = false;
@@ -205,6 +233,14 @@ struct hq_ctx {
   int nctl = 0;
   unsigned long long* d_clk = nullptr;  // phase cycles (HQ_SWEEP_PHASE_CLOCKS)
   int sweep_grid = 0;
+  // the finish of the log-det adjoint, laid out by its first call and again after a change of a
+  // hopping matrix: the eigenbases of K, the products' job lists, the results' buffer
+  char* d_adj = nullptr;
+  const double** d_eig = nullptr;      // per chain: its eigenvalues
+  long long* d_adj_off = nullptr;      // per chain: where its results start
+  double *d_adj_out = nullptr, *d_adj_logdet = nullptr;
+  size_t adj_doubles = 0;              // of all chains' results
+  HqGemmJob* adj_jobs[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   bool at_zero = false;         // stacks at tau = 0 (left empty, right full)
   bool at_beta = false;         // stacks at tau = beta
   bool initialised = false;
@@ -216,6 +252,7 @@ struct hq_ctx {
     if (d_lists) cudaFree(d_lists);
     if (d_ctl) cudaFree(d_ctl);
     if (d_clk) cudaFree(d_clk);
+    if (d_adj) cudaFree(d_adj);
     if (d_desc) cudaFree(d_desc);
     if (d_acc_all) cudaFree(d_acc_all);
     if (h_acc_all) cudaFreeHost(h_acc_all);
@@ -383,6 +420,87 @@ void build_jobs(hq_ctx* c) {
     std::tie(phase, dir, b, off, count) = t;
     c->jobs[std::make_tuple(phase, dir, b)] = {c->d_jobs + off, count};
   }
+}
+
+// The finish of the log-det adjoint: Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T with Q the eigenbasis of
+// K. Q and the eigenvalues are constants of the chains' hopping matrices (one copy per distinct
+// lattice and parameters, one per custom matrix); the five products are batched jobs over all chains.
+void build_adjoint(hq_ctx* c) {
+  size_t total = 0;
+  auto take = [&](size_t bytes) { const size_t o = total; total += align256(bytes); return o; };
+  std::map<std::tuple<int, double, double>, std::pair<size_t, size_t>> uniform;  // Q, w
+  std::vector<std::pair<size_t, size_t>> at(c->n);
+  std::vector<long long> off(c->n);
+  c->adj_doubles = 0;
+  for (int i = 0; i < c->n; ++i) {
+    const ChainHost& h = c->ch[i];
+    const size_t qb = size_t(h.N) * h.N * sizeof(double), wb = h.N * sizeof(double);
+    if (h.custom_hop) {
+      at[i].first = take(qb);
+      at[i].second = take(wb);
+    } else {
+      auto key = std::make_tuple(h.p.nl, h.p.nnt, h.p.mu);
+      if (!uniform.count(key)) {
+        const size_t q = take(qb);
+        uniform[key] = {q, take(wb)};
+      }
+      at[i] = uniform[key];
+    }
+    off[i] = (long long)c->adj_doubles;
+    c->adj_doubles += 2 + size_t(h.N) * h.N;
+  }
+  const size_t o_eig = take(c->n * sizeof(double*)), o_off = take(c->n * sizeof(long long));
+  const size_t o_out = take(c->adj_doubles * sizeof(double)), o_ld = take(c->n * sizeof(double));
+  size_t o_jobs[5];
+  for (auto& o : o_jobs) o = take(c->n * sizeof(HqGemmJob));
+  char* base = nullptr;
+  if (cudaMalloc(&base, total) != cudaSuccess) {
+    cudaGetLastError();
+    throw HqError(HQ_E_NOMEM, "hq_logdet_adjoint: no room for " + std::to_string(total) + " bytes");
+  }
+  try {
+    std::vector<double> w, Q;
+    auto put = [&](const std::pair<size_t, size_t>& o, const std::vector<double>& ww, const std::vector<double>& qq) {
+      HQ_CUDA(cudaMemcpy(base + o.first, qq.data(), qq.size() * sizeof(double), cudaMemcpyHostToDevice));
+      HQ_CUDA(cudaMemcpy(base + o.second, ww.data(), ww.size() * sizeof(double), cudaMemcpyHostToDevice));
+    };
+    for (auto& kv : uniform) {
+      int L;
+      double t, mu;
+      std::tie(L, t, mu) = kv.first;
+      w.resize(L * L);
+      Q.resize(size_t(L) * L * L * L);
+      lattice_eig(L, t, mu, w.data(), Q.data());
+      put(kv.second, w, Q);
+    }
+    std::vector<const double*> eig(c->n);
+    std::vector<HqGemmJob> jobs[5];
+    for (int i = 0; i < c->n; ++i) {
+      const ChainHost& h = c->ch[i];
+      if (h.custom_hop) put(at[i], h.eig_w, h.eig_Q);
+      eig[i] = reinterpret_cast<const double*>(base + at[i].second);
+      const double* q = reinterpret_cast<const double*>(base + at[i].first);
+      const HqChain& d = c->desc[i];
+      jobs[0].push_back(make_job(d.N, d.inv_expK, 0, d.W4, 0, d.W2));  // E^-1 D
+      jobs[1].push_back(make_job(d.N, q, 1, d.W2, 0, d.W3));           // Q^T E^-1 D
+      jobs[2].push_back(make_job(d.N, d.W3, 0, q, 0, d.W2));           // Q^T E^-1 D Q
+      jobs[3].push_back(make_job(d.N, q, 0, d.W3, 0, d.W2));           // Q (Phi o (.)^T)
+      jobs[4].push_back(make_job(d.N, d.W2, 0, q, 1, d.W3));           // Gamma
+    }
+    for (int k = 0; k < 5; ++k)
+      HQ_CUDA(cudaMemcpy(base + o_jobs[k], jobs[k].data(), jobs[k].size() * sizeof(HqGemmJob), cudaMemcpyHostToDevice));
+    HQ_CUDA(cudaMemcpy(base + o_eig, eig.data(), eig.size() * sizeof(double*), cudaMemcpyHostToDevice));
+    HQ_CUDA(cudaMemcpy(base + o_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice));
+  } catch (...) {
+    cudaFree(base);
+    throw;
+  }
+  c->d_adj = base;
+  c->d_eig = reinterpret_cast<const double**>(base + o_eig);
+  c->d_adj_off = reinterpret_cast<long long*>(base + o_off);
+  c->d_adj_out = reinterpret_cast<double*>(base + o_out);
+  c->d_adj_logdet = reinterpret_cast<double*>(base + o_ld);
+  for (int k = 0; k < 5; ++k) c->adj_jobs[k] = reinterpret_cast<HqGemmJob*>(base + o_jobs[k]);
 }
 
 // The persistent sweep's scheduling data: per chain {n_stab, estimated cycles of one interval}
@@ -893,6 +1011,13 @@ int hq_set_hopping(hq_ctx* c, int chain, const double* hop) {
   // exp(-+dt K) through the eigen-decomposition of the symmetric K
   std::vector<double> w, Q;
   jacobi_eig(N, h.K, w, Q);
+  h.eig_w = w;
+  h.eig_Q = Q;
+  if (c->d_adj) {
+    HQ_CUDA(cudaStreamSynchronize(c->stream));
+    cudaFree(c->d_adj);
+    c->d_adj = nullptr;
+  }
   std::vector<double> E(size_t(N) * N), Ei(size_t(N) * N), QE(size_t(N) * N), QEi(size_t(N) * N);
   for (int j = 0; j < N; ++j)
     for (int i = 0; i < N; ++i) {
@@ -1491,15 +1616,11 @@ int hq_download_fields_i8(hq_ctx* c, signed char* all) {
 
 int hq_logdet_adjoint(hq_ctx* c, double* out, double* logdet) {
   HQ_API_BEGIN
-  if (!c) throw HqError(HQ_E_INVALID, "null context");
+  if (!c || !out) throw HqError(HQ_E_INVALID, "null argument");
   if (!c->initialised || !c->at_zero) throw HqError(HQ_E_INVALID, "hq_logdet_adjoint: stacks must be at tau = 0");
   c->prof_next = 0;
-  // zero D (W4) and the scalar accumulators
-  for (int i = 0; i < c->n; ++i) {
-    const HqChain& d = c->desc[i];
-    HQ_CUDA(cudaMemsetAsync(d.W4, 0, size_t(d.N) * d.N * sizeof(double), c->stream));
-    HQ_CUDA(cudaMemsetAsync(d.acc + HQ_ACC_DMU, 0, 2 * sizeof(double), c->stream));
-  }
+  if (!c->d_adj) build_adjoint(c);
+  { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_adj_begin(c->d_desc, c->n, c->stream)); }
   // no-update up pass: wrap slice by slice, rebuild G from the stacks every pace slices
   // (the checkpoints), accumulate the adjoint contractions of every slice
   for (int b = 0; b < c->nstab_max; ++b) {
@@ -1515,62 +1636,17 @@ int hq_logdet_adjoint(hq_ctx* c, double* out, double* logdet) {
   // log|det(1 + U D Vt)| = sum log dmax + log|det(dmax^-1 U^T + dmin Vt)| from the full left stack
   run_jobs(c, PH_LOGDET, 0, 0);
   run_jobs(c, PH_LOGDET, 0, 1);
-  HQ_CUDA(cudaStreamSynchronize(c->stream));
-  size_t off = 0;
-  for (int i = 0; i < c->n; ++i) {
-    const HqChain& d = c->desc[i];
-    ChainHost& h = c->ch[i];
-    const int N = d.N;
-    const size_t NN = size_t(N) * N;
-    std::vector<double> D(NN), Wm(NN), Dl(N);
-    double acc[HQ_ACC_COUNT];
-    read_acc(c, i, acc);
-    HQ_CUDA(cudaMemcpy(D.data(), d.W4, NN * sizeof(double), cudaMemcpyDeviceToHost));
-    HQ_CUDA(cudaMemcpy(Wm.data(), d.W1, NN * sizeof(double), cudaMemcpyDeviceToHost));
-    HQ_CUDA(cudaMemcpy(Dl.data(), d.stackD + size_t(d.n_stab - 1) * N, N * sizeof(double), cudaMemcpyDeviceToHost));
-    // log-determinant (host LU with partial pivoting of the well-conditioned middle matrix)
-    double ld = 0.0;
-    for (int k = 0; k < N; ++k) ld += std::log(std::max(Dl[k], 1.0));
-    {
-      std::vector<double> M = Wm;
-      for (int k = 0; k < N; ++k) {
-        int p = k;
-        for (int r = k + 1; r < N; ++r)
-          if (std::fabs(M[r + size_t(k) * N]) > std::fabs(M[p + size_t(k) * N])) p = r;
-        if (p != k)
-          for (int j = 0; j < N; ++j) std::swap(M[k + size_t(j) * N], M[p + size_t(j) * N]);
-        const double pv = M[k + size_t(k) * N];
-        ld += std::log(std::fabs(pv));
-        for (int r = k + 1; r < N; ++r) {
-          const double f = M[r + size_t(k) * N] / pv;
-          for (int j = k + 1; j < N; ++j) M[r + size_t(j) * N] -= f * M[k + size_t(j) * N];
-        }
-      }
-    }
-    if (logdet) logdet[i] = ld;
-    // Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T, Phi = divided differences of exp(-dt lambda)
-    std::vector<double> w, Q;
-    jacobi_eig(N, h.K, w, Q);
-    std::vector<double> Einv(NN), M1(NN), M2(NN), Mt(NN), P(NN), G1(NN), Gam(NN);
-    for (int j = 0; j < N; ++j)
-      for (int i2 = 0; i2 < N; ++i2) M1[i2 + size_t(j) * N] = Q[i2 + size_t(j) * N] * std::exp(h.dt * w[j]);
-    host_gemm(N, M1.data(), false, Q.data(), true, Einv.data());  // E^-1 = exp(+dt K)
-    host_gemm(N, Einv.data(), false, D.data(), false, M1.data());  // M = E^-1 D
-    host_gemm(N, Q.data(), true, M1.data(), false, M2.data());     // Q^T M
-    host_gemm(N, M2.data(), false, Q.data(), false, Mt.data());    // Q^T M Q
-    for (int j = 0; j < N; ++j)
-      for (int i2 = 0; i2 < N; ++i2) {
-        const double fi = std::exp(-h.dt * w[i2]), fj = std::exp(-h.dt * w[j]);
-        const double dd = std::fabs(w[i2] - w[j]) > 1e-10 ? (fi - fj) / (w[i2] - w[j]) : -h.dt * 0.5 * (fi + fj);
-        P[i2 + size_t(j) * N] = dd * Mt[j + size_t(i2) * N];
-      }
-    host_gemm(N, Q.data(), false, P.data(), false, G1.data());
-    host_gemm(N, G1.data(), false, Q.data(), true, Gam.data());
-    out[off + 0] = acc[HQ_ACC_DMU];
-    out[off + 1] = acc[HQ_ACC_DALPHA];
-    std::memcpy(out + off + 2, Gam.data(), NN * sizeof(double));
-    off += 2 + NN;
+  { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_logdet(c->d_desc, c->n, c->d_adj_logdet, c->Nmax, c->resident, c->stream)); }
+  // Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T, Phi = divided differences of exp(-dt lambda)
+  for (int k = 0; k < 5; ++k) {
+    { ProfScope ps(c, PC_GEMM); HQ_CUDA(hq::launch_gemm(c->adj_jobs[k], c->n, c->Nmax, c->Nmax, c->stream)); }
+    if (k == 2) HQ_CUDA(hq::launch_adj_divided(c->d_desc, c->n, c->d_eig, c->stream));
   }
+  HQ_CUDA(hq::launch_adj_gather(c->d_desc, c->n, c->d_adj_off, c->d_adj_out, c->stream));
+  HQ_CUDA(cudaMemcpyAsync(out, c->d_adj_out, c->adj_doubles * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  if (logdet)
+    HQ_CUDA(cudaMemcpyAsync(logdet, c->d_adj_logdet, c->n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  HQ_CUDA(cudaStreamSynchronize(c->stream));
   // the pass left the stacks at tau = beta
   c->at_zero = false;
   c->at_beta = true;

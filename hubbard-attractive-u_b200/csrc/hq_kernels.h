@@ -59,5 +59,11 @@ cudaError_t launch_sweep(const HqChain* chains, int nchains, const int2* cinfo, 
                          unsigned long long* clk, int grid, int Nmax, int kmax, cudaStream_t st);
 const void* fn_sweep();
 cudaError_t launch_adj_interval(const HqChain* chains, int n, int b, int Nmax, bool resident, cudaStream_t st);
+// the finish of the log-det adjoint: log|det| per chain (out), the Daleckii-Krein factor between the
+// products of the eigenbasis of K, the results in the caller's layout
+cudaError_t launch_adj_begin(const HqChain* chains, int n, cudaStream_t st);
+cudaError_t launch_logdet(const HqChain* chains, int n, double* out, int Nmax, bool resident, cudaStream_t st);
+cudaError_t launch_adj_divided(const HqChain* chains, int n, const double* const* eig, cudaStream_t st);
+cudaError_t launch_adj_gather(const HqChain* chains, int n, const long long* off, double* out, cudaStream_t st);
 cudaError_t launch_adj_last(const HqChain* chains, int n, int b, cudaStream_t st);
 }  // namespace hq

@@ -161,3 +161,32 @@ def test_autograd_function_gradcheck(hq, oracle):
     o.set_fields(fields)
     ld = float(f(t, mu, u).detach())
     assert abs(ld - o.logdet()) <= 1e-9 * max(1.0, abs(ld))
+
+
+@pytest.mark.parametrize("L,chains", [(1, 1), (2, 2), (3, 3), (5, 2), (8, 2), (13, 1)])
+def test_adjoint_finish_at_the_edges(hq, oracle, L, chains):
+    """Log-determinant and gradients for uniform hoppings (closed-form eigenbasis of K, degenerate
+    levels) from one site to a lattice beyond one SM, beside a second call after set_hopping of
+    unequal bonds (numerical eigenbasis), against the oracle at the bounds of the other tests."""
+    nt, beta, mu, u = 6, 0.6, -0.2, 4.0
+    cfg = dict(nl=L, u=u, mu=mu, beta=beta, nt=nt, stabilization_pace=4)
+    e = hq.Engine([dict(cfg, seed=c) for c in range(chains)])
+    fields = stream_fields(oracle, L, nt, 5, chains)
+    r = np.random.RandomState(1).uniform(0.7, 1.3, (L * L, L * L))
+    for hop in (nn_hop(L), nn_hop(L) * (r + r.T) / 2):
+        for c in range(chains):
+            if not np.array_equal(hop, nn_hop(L)):
+                e.set_hopping(c, hop)
+            e.set_fields(c, fields[c])
+        e.init()
+        ld, grads = e.logdet_adjoint()
+        for c in range(chains):
+            o = oracle.OracleChain(L, u=u, mu=mu, beta=beta, nt=nt, pace=4, seed=1, custom_hop=hop)
+            o.set_fields(fields[c])
+            o.init()
+            dmu, dal, dK = o.logdet_grad()
+            assert abs(ld[c] - o.logdet()) <= 1e-9 * max(1.0, abs(ld[c]))
+            assert abs(grads[c][0] - dmu) <= 1e-8 * max(1.0, abs(dmu))
+            assert abs(grads[c][1] - dal) <= 1e-8 * max(1.0, abs(dal))
+            assert np.abs(grads[c][2] - dK).max() <= 1e-8 * max(1.0, np.abs(dK).max())
+    e.close()
