@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -595,17 +596,20 @@ Cur cur(hq_ctx* c) {
   return {c->d_desc + c->cur_c0, c->cur_n, c->cur_st};
 }
 
-void run_jobs(hq_ctx* c, int phase, int dir, int b) {
+// the products of up to three phases (none depending on another) of the current chain group in one launch
+void run_jobs(hq_ctx* c, std::initializer_list<int> phases, int dir, int b) {
   ProfScope ps(c, PC_GEMM);
-  auto it = c->jobs.find(std::make_tuple(phase, dir, b));
-  if (it == c->jobs.end()) throw HqError(HQ_E_INVALID, "internal: missing job list");
-  if (c->cur_st) {
-    // per-chain phases hold one job per chain, in chain order
+  const Cur g = cur(c);
+  hq::HqGemmLists lists{};
+  int k = 0;
+  for (int phase : phases) {
+    auto it = c->jobs.find(std::make_tuple(phase, dir, b));
+    if (it == c->jobs.end()) throw HqError(HQ_E_INVALID, "internal: missing job list");
+    // the phases hold one job per chain, in chain order
     if (it->second.second != c->n) throw HqError(HQ_E_INVALID, "internal: job list is not per chain");
-    HQ_CUDA(hq::launch_gemm(it->second.first + c->cur_c0, c->cur_n, c->Nmax, c->Nmax, c->cur_st));
-  } else {
-    HQ_CUDA(hq::launch_gemm(it->second.first, it->second.second, c->Nmax, c->Nmax, c->stream));
+    lists.l[k++] = it->second.first + (g.d - c->d_desc);
   }
+  HQ_CUDA(hq::launch_gemm(lists, k, g.n, c->Nmax, c->Nmax, g.st));
 }
 
 void upload_desc(hq_ctx* c) {
@@ -626,8 +630,8 @@ bool interval_on_clusters(hq_ctx* c) {
   return true;
 }
 
-// one stack push of interval b: bchain -> UDV -> cumulative Vt
-void push_step(hq_ctx* c, int dir_kernel, int dir_jobs, int b) {
+// one stack push of interval b: bchain -> UDV; the cumulative Vt is left to the next products
+void push_factor(hq_ctx* c, int dir_kernel, int b) {
   const Cur g = cur(c);
   {
     ProfScope ps(c, PC_BCHAIN);
@@ -636,16 +640,22 @@ void push_step(hq_ctx* c, int dir_kernel, int dir_jobs, int b) {
   }
   const int side = (dir_kernel == HQ_DOWN) ? 1 : 0;
   { ProfScope ps(c, PC_UDT); HQ_CUDA(hq::launch_udt(g.d, g.n, side, b, c->Nmax, c->resident, g.st)); }
-  run_jobs(c, PH_PUSH, dir_jobs, b);
 }
 
-void builder_equaltime(hq_ctx* c, int dir_jobs, int b) {
+// W1^-1 of the G builder after the push of interval b; with_push: the push's own product (the
+// cumulative Vt) rides in the launch of the first builder product, which does not read it
+void builder_inverse(hq_ctx* c, int dir_jobs, int b, bool with_push) {
   const Cur g = cur(c);
-  run_jobs(c, PH_B1, dir_jobs, b);
-  run_jobs(c, PH_B2, dir_jobs, b);
+  if (with_push) run_jobs(c, {PH_PUSH, PH_B1}, dir_jobs, b);
+  else run_jobs(c, {PH_B1}, dir_jobs, b);
+  run_jobs(c, {PH_B2}, dir_jobs, b);
   { ProfScope ps(c, PC_INVERT); HQ_CUDA(hq::launch_invert(g.d, g.n, b, 0, c->Nmax, c->resident, g.st)); }
-  run_jobs(c, PH_B3, dir_jobs, b);
-  run_jobs(c, PH_B4, dir_jobs, b);
+}
+
+void builder_equaltime(hq_ctx* c, int dir_jobs, int b, bool with_push) {
+  builder_inverse(c, dir_jobs, b, with_push);
+  run_jobs(c, {PH_B3}, dir_jobs, b);
+  run_jobs(c, {PH_B4}, dir_jobs, b);
 }
 
 // Runs body() once per chain group, each group on its own stream forked from the main
@@ -696,8 +706,8 @@ void issue_sweep(hq_ctx* c, int dir, int flags) {
           ProfScope ps(c, PC_INTERVAL);
           HQ_CUDA(hq::launch_interval(gr.d, gr.n, dir, b, kf, c->Nmax, c->kmax_max, c->resident, gr.st));
         }
-        push_step(c, dir, dir, b);
-        builder_equaltime(c, dir, b);
+        push_factor(c, dir, b);
+        builder_equaltime(c, dir, b, true);
         if (kf & (HQ_F_MEASURE | HQ_F_SNAPSHOT)) { ProfScope ps(c, PC_MEASURE); HQ_CUDA(hq::launch_measure(gr.d, gr.n, dir, b, kf, gr.st)); }
       }
     });
@@ -705,15 +715,10 @@ void issue_sweep(hq_ctx* c, int dir, int flags) {
     { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_start(c->d_desc, c->n, c->stream)); }
     for (int b = 0; b < c->nstab_max; ++b) {
       { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_slices(c->d_desc, c->n, b, kf, c->Nmax, c->resident, c->stream)); }
-      push_step(c, HQ_UP, 3, b);
-      run_jobs(c, PH_B1, 3, b);
-      run_jobs(c, PH_B2, 3, b);
-      { ProfScope ps(c, PC_INVERT); HQ_CUDA(hq::launch_invert(c->d_desc, c->n, b, 0, c->Nmax, c->resident, c->stream)); }
-      run_jobs(c, PH_B3, 3, b);   // W2 = Y = T1^-1 dlmax^-1 U_L^T
-      run_jobs(c, PH_D3, 3, b);   // W3 = G(t,t)
-      run_jobs(c, PH_D4, 3, b);   // W5 = T1^-1 dlmin Vt_L
-      run_jobs(c, PH_D5, 3, b);   // W0 = G(t,0)
-      run_jobs(c, PH_D6, 3, b);   // W4 = G(0,t)
+      push_factor(c, HQ_UP, b);
+      builder_inverse(c, 3, b, true);
+      run_jobs(c, {PH_B3, PH_D4}, 3, b);         // W2 = Y = T1^-1 dlmax^-1 U_L^T, W5 = T1^-1 dlmin Vt_L
+      run_jobs(c, {PH_D3, PH_D5, PH_D6}, 3, b);  // W3 = G(t,t), W0 = G(t,0), W4 = G(0,t)
       { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_commit(c->d_desc, c->n, b, c->stream)); }
       { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_store(c->d_desc, c->n, b, c->stream)); }
       { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_measure(c->d_desc, c->n, b, 0, c->stream)); }
@@ -1134,9 +1139,12 @@ int hq_init_stacks_and_g(hq_ctx* c) {
   nstabs.erase(std::unique(nstabs.begin(), nstabs.end()), nstabs.end());
   in_groups(c, [&] {
     // src/dqmc_core.cpp:67-87: right stack from t = nt down to 1 with B^T, push every pace
-    for (int b = 0; b < c->nstab_max; ++b) push_step(c, HQ_DOWN, 2, b);
+    for (int b = 0; b < c->nstab_max; ++b) {
+      push_factor(c, HQ_DOWN, b);
+      run_jobs(c, {PH_PUSH}, 2, b);
+    }
     // src/dqmc_core.cpp:89-97: G(0,0) from (empty left, full right)
-    if (nstabs.size() == 1) builder_equaltime(c, 2, nstabs[0] - 1);
+    if (nstabs.size() == 1) builder_equaltime(c, 2, nstabs[0] - 1, false);
   });
   if (nstabs.size() > 1) {
     for (int ns : nstabs) {
@@ -1144,7 +1152,7 @@ int hq_init_stacks_and_g(hq_ctx* c) {
       std::vector<HqChain> saved = c->desc;
       for (int i = 0; i < c->n; ++i) c->desc[i].active = (c->ch[i].n_stab == ns) ? 1 : 0;
       upload_desc(c);
-      builder_equaltime(c, 2, ns - 1);
+      builder_equaltime(c, 2, ns - 1, false);
       HQ_CUDA(cudaStreamSynchronize(c->stream));
       c->desc = saved;
       upload_desc(c);
@@ -1625,17 +1633,13 @@ int hq_logdet_adjoint(hq_ctx* c, double* out, double* logdet) {
   // (the checkpoints), accumulate the adjoint contractions of every slice
   for (int b = 0; b < c->nstab_max; ++b) {
     { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_adj_interval(c->d_desc, c->n, b, c->Nmax, c->resident, c->stream)); }
-    push_step(c, HQ_UP, HQ_UP, b);
-    run_jobs(c, PH_B1, HQ_UP, b);
-    run_jobs(c, PH_B2, HQ_UP, b);
-    { ProfScope ps(c, PC_INVERT); HQ_CUDA(hq::launch_invert(c->d_desc, c->n, b, 0, c->Nmax, c->resident, c->stream)); }
-    run_jobs(c, PH_B3, HQ_UP, b);
-    run_jobs(c, PH_B4, HQ_UP, b);
+    push_factor(c, HQ_UP, b);
+    builder_equaltime(c, HQ_UP, b, true);
     { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_adj_last(c->d_desc, c->n, b, c->stream)); }
   }
   // log|det(1 + U D Vt)| = sum log dmax + log|det(dmax^-1 U^T + dmin Vt)| from the full left stack
-  run_jobs(c, PH_LOGDET, 0, 0);
-  run_jobs(c, PH_LOGDET, 0, 1);
+  run_jobs(c, {PH_LOGDET}, 0, 0);
+  run_jobs(c, {PH_LOGDET}, 0, 1);
   { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_logdet(c->d_desc, c->n, c->d_adj_logdet, c->Nmax, c->resident, c->stream)); }
   // Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T, Phi = divided differences of exp(-dt lambda)
   for (int k = 0; k < 5; ++k) {

@@ -53,15 +53,17 @@ __device__ __forceinline__ void g_stage(const double* X, int ldx, bool kmaj, int
   }
 }
 
+// Up to three job lists of n jobs each in one launch (products that do not depend on each other: the
+// push with the first builder product, the displaced builder's in two rounds), so that a sweep's
+// interval has four instead of five of these launches and a dynamic one five instead of eight.
 __global__ void __launch_bounds__(kGWarps * 32, 4)
-k_gemm(const HqGemmJob* __restrict__ jobs, int njobs, int tiles_n) {
+k_gemm(HqGemmLists lists, int njobs, int tiles_n) {
   __shared__ __align__(16) double sA[2][kGStage];
   __shared__ __align__(16) double sB[2][kGStage];
   __shared__ double sK[2][kGKc];
   __shared__ double red[32];
-  const int jb = blockIdx.y;
-  if (jb >= njobs) return;
-  const HqGemmJob J = jobs[jb];
+  const int li = blockIdx.y / njobs, jb = blockIdx.y - li * njobs;
+  const HqGemmJob J = (li == 0 ? lists.l[0] : (li == 1 ? lists.l[1] : lists.l[2]))[jb];
   if (!J.active) return;
   const int m0 = (blockIdx.x / tiles_n) * kGT, n0 = (blockIdx.x % tiles_n) * kGT;
   if (m0 >= J.M || n0 >= J.Nc) return;
@@ -111,8 +113,30 @@ k_gemm(const HqGemmJob* __restrict__ jobs, int njobs, int tiles_n) {
     __syncthreads();
   }
   cp_async_wait<0>();
-  // epilogue: alpha, row / column scalings, beta, wrap-error maximum
+  // epilogue: alpha, row / column scalings, beta, wrap-error maximum. A thread's two rows and six
+  // columns take eight scalings (divisions among them) instead of one pair per element, and the old
+  // values are loaded before the first store.
   double emax = -INFINITY;
+  double rsv[2], csv[6], old[3][4];
+  const bool load_old = J.beta != 0.0 || J.epi == 1;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int gm = m0 + wm + g + 8 * h;
+    rsv[h] = gm < J.M ? vscale(J.rs, J.rs_mode, gm) : 0.0;
+  }
+#pragma unroll
+  for (int h = 0; h < 6; ++h) {
+    const int gn = n0 + wn + (h >> 1) * 8 + 2 * q + (h & 1);
+    csv[h] = gn < J.Nc ? vscale(J.cs, J.cs_mode, gn) : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int gm = m0 + wm + g + ((e & 2) ? 8 : 0);
+      const int gn = n0 + wn + j * 8 + 2 * q + (e & 1);
+      old[j][e] = (load_old && gm < J.M && gn < J.Nc) ? J.C[gm + (size_t)gn * J.ldc] : 0.0;
+    }
 #pragma unroll
   for (int j = 0; j < 3; ++j)
 #pragma unroll
@@ -120,12 +144,10 @@ k_gemm(const HqGemmJob* __restrict__ jobs, int njobs, int tiles_n) {
       const int gm = m0 + wm + g + ((e & 2) ? 8 : 0);
       const int gn = n0 + wn + j * 8 + 2 * q + (e & 1);
       if (gm < J.M && gn < J.Nc) {
-        double v = J.alpha * acc[j][e] * vscale(J.rs, J.rs_mode, gm) * vscale(J.cs, J.cs_mode, gn);
-        double* cp = J.C + gm + (size_t)gn * J.ldc;
-        const double old = (J.beta != 0.0 || J.epi == 1) ? *cp : 0.0;
-        if (J.beta != 0.0) v = fma(J.beta, old, v);
-        if (J.epi == 1) emax = fmax(emax, v - old);
-        *cp = v;
+        double v = J.alpha * acc[j][e] * rsv[e >> 1] * csv[2 * j + (e & 1)];
+        if (J.beta != 0.0) v = fma(J.beta, old[j][e], v);
+        if (J.epi == 1) emax = fmax(emax, v - old[j][e]);
+        J.C[gm + (size_t)gn * J.ldc] = v;
       }
     }
   if (J.epi == 1 && J.err_out) {
@@ -134,12 +156,15 @@ k_gemm(const HqGemmJob* __restrict__ jobs, int njobs, int tiles_n) {
   }
 }
 
-cudaError_t launch_gemm(const HqGemmJob* jobs, int njobs, int Mmax, int Nmax, cudaStream_t st) {
-  if (njobs <= 0) return cudaSuccess;
+cudaError_t launch_gemm(const HqGemmLists& lists, int nlists, int njobs, int Mmax, int Nmax, cudaStream_t st) {
+  if (njobs <= 0 || nlists <= 0) return cudaSuccess;
   const int tm = (Mmax + kGT - 1) / kGT, tn = (Nmax + kGT - 1) / kGT;
-  dim3 grid(tm * tn, njobs);
-  k_gemm<<<grid, kGWarps * 32, 0, st>>>(jobs, njobs, tn);
+  dim3 grid(tm * tn, njobs * nlists);
+  k_gemm<<<grid, kGWarps * 32, 0, st>>>(lists, njobs, tn);
   return cudaGetLastError();
+}
+cudaError_t launch_gemm(const HqGemmJob* jobs, int njobs, int Mmax, int Nmax, cudaStream_t st) {
+  return launch_gemm(HqGemmLists{{jobs, nullptr, nullptr}}, 1, njobs, Mmax, Nmax, st);
 }
 
 }  // namespace hq

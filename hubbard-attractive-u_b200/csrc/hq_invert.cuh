@@ -20,42 +20,42 @@ namespace hq {
 //  gather on the way out. Failure (zero pivot / non-finite) sets acc[STATUS].
 // ---------------------------------------------------------------------------------
 
-// x[r / 32] (r warp-uniform) without an indexed access: written as a C++ select chain the
-// compiler folds it back into x[r / 32], which moves x to local memory; selp keeps it in
-// registers
+// x[r / 32] (r warp-uniform) without an indexed access, as a tree of selections on the bits of r / 32:
+// written as a C++ select chain the compiler folds it back into x[r / 32], which moves x to local
+// memory; selp keeps it in registers
+__device__ __forceinline__ double sel2(double a, double b, int bit) {
+  double v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f64 %0, %2, %1, p;\n\t}" : "=d"(v) : "d"(a), "d"(b), "r"(bit));
+  return v;
+}
 template <int RPL>
 __device__ __forceinline__ double slot_at(const double (&x)[RPL], int r) {
+  static_assert(RPL >= 1 && RPL <= 8, "three levels");
   const int t = r >> 5;
-  double v = 0.0;
-#pragma unroll
-  for (int i = 0; i < RPL; ++i)
-    asm("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %2, %3;\n\tselp.f64 %0, %1, %0, p;\n\t}" : "+d"(v) : "d"(x[i]), "r"(t), "r"(i));
-  return v;
+  auto lo4 = [&](int o) {  // of x[o .. o + 3]
+    const double a = o + 1 < RPL ? sel2(x[o], x[o + 1 < RPL ? o + 1 : 0], t & 1) : x[o];
+    if (o + 2 >= RPL) return a;
+    const double b = o + 3 < RPL ? sel2(x[o + 2 < RPL ? o + 2 : 0], x[o + 3 < RPL ? o + 3 : 0], t & 1) : x[o + 2 < RPL ? o + 2 : 0];
+    return sel2(a, b, t & 2);
+  };
+  if constexpr (RPL <= 4) return lo4(0);
+  else return sel2(lo4(0), lo4(4), t & 4);
 }
 
-// the same for five slots as a tree of depth 3 (bits 0, 1 and 2 of r / 32)
-template <>
-__device__ __forceinline__ double slot_at<5>(const double (&x)[5], int r) {
-  const int t = r >> 5;
-  double a, b, c, v;
-  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f64 %0, %2, %1, p;\n\t}" : "=d"(a) : "d"(x[0]), "d"(x[1]), "r"(t & 1));
-  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f64 %0, %2, %1, p;\n\t}" : "=d"(b) : "d"(x[2]), "d"(x[3]), "r"(t & 1));
-  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f64 %0, %2, %1, p;\n\t}" : "=d"(c) : "d"(a), "d"(b), "r"(t & 2));
-  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f64 %0, %2, %1, p;\n\t}" : "=d"(v) : "d"(c), "d"(x[4]), "r"(t & 4));
-  return v;
-}
-
-// pivot k of a register-resident Gauss-Jordan panel, by the warp that holds column k:
+// Pivot k of a register-resident Gauss-Jordan panel, by the warp that holds column k:
 // partial pivoting (largest |A[r][k]|, r >= k, smallest index among equals), row swap in
-// this column, the multipliers into fcol, the inverse's column k into x, and perm / pinv
+// this column, the multipliers into fcol, the inverse's column k into x, and perm / pinv.
+// The chain of a pivot: the lane's candidate by a pairwise tree over its slots, three redux steps
+// (high word of |x|, low word, smallest row), the pivot's value from its lane's candidate. Every lane
+// stores (padding rows into the padding of fcol), so that nothing branches.
 template <int RPL>
 __device__ __forceinline__ void gj_pivot_reg(double (&x)[RPL], int k, int N, double* fcol, double* pinv_out,
                                              int* perm, double* status) {
   const int lane = threadIdx.x & 31;
+  const double vk = __shfl_sync(0xffffffffu, slot_at<RPL>(x, k), k & 31);
   // the lane's candidate: the largest |x[t]| over its rows r >= k, the smallest such row among
-  // equals; rows out of range and NaNs are (-1, N) and never win. A pairwise tree over the slots
-  // (depth 3 for five) gives the same pair as a scan in row order.
-  double cv[RPL];
+  // equals; rows out of range and NaNs are (-1, N) and never win
+  double cv[RPL], cx[RPL];
   int cr[RPL];
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
@@ -64,6 +64,7 @@ __device__ __forceinline__ void gj_pivot_reg(double (&x)[RPL], int k, int N, dou
     const bool ok = r >= k && r < N && v == v;
     cv[t] = ok ? v : -1.0;
     cr[t] = ok ? r : N;
+    cx[t] = x[t];
   }
 #pragma unroll
   for (int w = 1; w < RPL; w *= 2)
@@ -72,48 +73,39 @@ __device__ __forceinline__ void gj_pivot_reg(double (&x)[RPL], int k, int N, dou
       const bool tb = cv[t + w] > cv[t] || (cv[t + w] == cv[t] && cr[t + w] < cr[t]);
       cv[t] = tb ? cv[t + w] : cv[t];
       cr[t] = tb ? cr[t + w] : cr[t];
+      cx[t] = tb ? cx[t + w] : cx[t];
     }
-  double best = cv[0];
-  int bi = cr[0];
-  // warp argmax with three redux steps on the bit pattern of |x| (monotonic for non-negative
-  // doubles; NaNs were skipped by the lane-local search): the high word, then the low word
-  // among the lanes holding the maximum, then the smallest row among those
-  {
-    const unsigned long long bb = best < 0.0 ? 0ull : (unsigned long long)__double_as_longlong(best);
-    const unsigned hi = (unsigned)(bb >> 32), lo = (unsigned)bb;
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-    bi = (int)__reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? (unsigned)bi : 0xffffffffu);
-    best = __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
-  }
-  const double vk = __shfl_sync(0xffffffffu, slot_at<RPL>(x, k), k & 31);
-  const double vb = __shfl_sync(0xffffffffu, slot_at<RPL>(x, bi), bi & 31);
-  const bool ok = (best > 0.0) && isfinite(best);
-  const double pinv = ok ? __drcp_rn(vb) : 0.0;  // = 1 / vb, correctly rounded
+  // the bit pattern of |x| orders non-negative doubles
+  const unsigned long long bb = cv[0] < 0.0 ? 0ull : (unsigned long long)__double_as_longlong(cv[0]);
+  const unsigned hi = (unsigned)(bb >> 32), lo = (unsigned)bb;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const int bi = (int)__reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? (unsigned)cr[0] : 0xffffffffu);
+  const double vb = __shfl_sync(0xffffffffu, cx[0], bi & 31);  // row bi is the candidate of its lane
+  const bool ok = (mh | ml) != 0u && isfinite(vb);
+  const double pinv = ok ? reciprocal(vb) : 0.0;
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
     const int r = lane + 32 * t;
-    double v = (r == k) ? vb : ((r == bi) ? vk : x[t]);
-    if (r < N) fcol[r] = v;
+    const double v = (r == k) ? vb : ((r == bi) ? vk : x[t]);
+    fcol[r] = v;
     x[t] = (r == k) ? pinv : -v * pinv;
   }
-  if (lane == 0) {
-    perm[k] = bi;
-    *pinv_out = pinv;
-    if (!ok) *status = 1.0;
-  }
+  perm[k] = bi;  // every lane the same values
+  *pinv_out = pinv;
+  if (!ok) *status = 1.0;
 }
 
 // Gauss-Jordan on the panel columns [p0, p0 + nb) of A (all rows), N <= 32 RPL: the panel's
 // columns are held in registers, CPW per warp by kGJ / CPW warps (warp w holds columns
 // p0 + w + i kGJ / CPW); the owner of column k+1 takes pivot k+1 right after its own elimination
 // step for pivot k, so one block barrier separates pivots. Multipliers and the reciprocal pivot
-// are double-buffered by pivot parity (fcol: 2N doubles, pv: 2).
+// are double-buffered by pivot parity (fcol: 64 RPL doubles, pv: 2).
 template <int RPL, int CPW>
 __device__ void gj_panel_reg(double* A, int ld, int N, int p0, int nb, int* perm, double* fcol, double* pv,
                              double* status) {
   constexpr int NWP = kGJ / CPW;  // warps that hold panel columns
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index();
   int col[CPW];
   bool own[CPW];
   double x[CPW][RPL];
@@ -127,6 +119,7 @@ __device__ void gj_panel_reg(double* A, int ld, int N, int p0, int nb, int* perm
       x[i][t] = (own[i] && r < N) ? A[r + (size_t)col[i] * ld] : 0.0;
     }
   }
+  constexpr int FS = 32 * RPL;
   if (warp == 0) gj_pivot_reg<RPL>(x[0], p0, N, fcol, pv, perm, status);
   __syncthreads();
   for (int q = 0; q < nb; ++q) {
@@ -136,7 +129,7 @@ __device__ void gj_panel_reg(double* A, int ld, int N, int p0, int nb, int* perm
       if (own[i] && col[i] != k) {
         const int bi = perm[k];
         const double pinv = pv[par];
-        const double* f = fcol + par * N;
+        const double* f = fcol + par * FS;
         // row swap k <-> bi in this column, then row k scaled by the pivot's reciprocal
         const double vk = __shfl_sync(0xffffffffu, slot_at<RPL>(x[i], k), k & 31);
         const double vb = __shfl_sync(0xffffffffu, slot_at<RPL>(x[i], bi), bi & 31);
@@ -145,10 +138,10 @@ __device__ void gj_panel_reg(double* A, int ld, int N, int p0, int nb, int* perm
         for (int t = 0; t < RPL; ++t) {
           const int r = lane + 32 * t;
           const double v = (r == bi) ? vk : x[i][t];
-          x[i][t] = (r == k) ? u : ((r < N) ? fma(-f[r < N ? r : 0], u, v) : v);
+          x[i][t] = (r == k) ? u : fma(-f[r], u, v);  // padding rows hold any values
         }
         if (col[i] == k + 1 && q + 1 < nb)
-          gj_pivot_reg<RPL>(x[i], k + 1, N, fcol + (par ^ 1) * N, pv + (par ^ 1), perm, status);
+          gj_pivot_reg<RPL>(x[i], k + 1, N, fcol + (par ^ 1) * FS, pv + (par ^ 1), perm, status);
       }
     }
     __syncthreads();
@@ -183,12 +176,17 @@ __device__ __forceinline__ void invert_body(const HqChain& ch, int which, bool r
   double* Bf = p; p += (size_t)ldp * kGJ;   // kGJ x N, row-major
   int* perm = reinterpret_cast<int*>(p);
   int* gidx = perm + N;
-  double* fcol = reinterpret_cast<double*>(gidx + N);  // 2 N multipliers (register panel)
+  double* fcol = reinterpret_cast<double*>(gidx + N);  // 64 ceil(N / 32) multipliers (register panel)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __syncthreads();
   for (int p0 = 0; p0 < N; p0 += kGJ) {
     const int nb = min(kGJ, N - p0);
-    if (N <= 160) gj_panel_reg<5, CPW>(A, ld, N, p0, nb, perm, fcol, pv, ch.acc + HQ_ACC_STATUS);
+    double* status = ch.acc + HQ_ACC_STATUS;
+    if (N <= 32) gj_panel_reg<1, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (N <= 64) gj_panel_reg<2, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (N <= 96) gj_panel_reg<3, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (N <= 128) gj_panel_reg<4, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (N <= 160) gj_panel_reg<5, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
     else for (int q = 0; q < nb; ++q) {
       const int k = p0 + q;
       if (warp == 0) {

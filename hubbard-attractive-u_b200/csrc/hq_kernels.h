@@ -20,6 +20,9 @@ cudaError_t launch_interval(const HqChain* chains, int n, int dir, int b, int fl
 cudaError_t launch_bchain(const HqChain* chains, int n, int dir, int b, int Nmax, bool resident, cudaStream_t st);
 cudaError_t launch_udt(const HqChain* chains, int n, int side, int b, int Nmax, bool resident, cudaStream_t st);
 cudaError_t launch_invert(const HqChain* chains, int n, int b, int which, int Nmax, bool resident, cudaStream_t st);
+// the jobs of up to three lists of njobs each, in one launch (none may depend on another)
+struct HqGemmLists { const HqGemmJob* l[3]; };
+cudaError_t launch_gemm(const HqGemmLists& lists, int nlists, int njobs, int Mmax, int Nmax, cudaStream_t st);
 cudaError_t launch_gemm(const HqGemmJob* jobs, int njobs, int Mmax, int Nmax, cudaStream_t st);
 cudaError_t launch_measure(const HqChain* chains, int n, int dir, int b, int flags, cudaStream_t st);
 cudaError_t launch_dyn_start(const HqChain* chains, int n, cudaStream_t st);

@@ -59,17 +59,6 @@ __device__ __forceinline__ double reference_ratio(double gii, double dl) {
   return __ddiv_rn(__dmul_rn(a, a), __dadd_rn(1.0, dl));
 }
 
-// 1 / x, correctly rounded for the walk's arguments (normal numbers): the hardware's approximation
-// (relative error below 2^-23) and two Newton steps y + y (1 - x y), whose FMA residuals leave 2^-92
-// before the last rounding. Without the range checks and the branch of the intrinsic, whose value
-// it has, the sites of a block are one stretch of straight code.
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
 // The walk of the nb <= 16 sites [b0, b0 + nb) by one warp. Lane 8 rg + cg holds the entries
 // (4 rg + a, 2 cg + b), a < 4, b < 2, of g: a step needs column s at the lane's four rows, row s at its
 // two columns and the diagonal entry, 7 shuffles. Entries of rows and columns already visited are

@@ -128,7 +128,7 @@ k_sweep(const HqChain* __restrict__ chains, int nchains, const int2* __restrict_
   __shared__ double red[96];
   __shared__ double pv[2];
   __shared__ int2 s_item;
-  __shared__ HqGemmJob job;
+  __shared__ HqGemmJob jobs[5];
   const int side = (dir == HQ_DOWN) ? 1 : 0;
   // phase cycles (HQ_F_PHASE_CLOCKS), taken by thread 0 after the barrier that ends a phase
   const bool clocks = (flags & HQ_F_PHASE_CLOCKS) && clk;
@@ -159,6 +159,15 @@ k_sweep(const HqChain* __restrict__ chains, int nchains, const int2* __restrict_
     __syncthreads();
     if (s_item.x < 0) break;
     const int c = s_item.x, b = s_item.y, N = ch.N;
+    // the item's five builder jobs, while G is on its way (read barriers later)
+    {
+      static_assert(sizeof(HqGemmJob) == 128, "16 words of 8 bytes");
+      const int w = (int)threadIdx.x - 32;
+      if (w >= 0 && w < 80) {
+        const HqGemmJob* src = lists[((size_t)dir * nstab_max + b) * 5 + w / 16] + c;
+        reinterpret_cast<unsigned long long*>(jobs + w / 16)[w % 16] = reinterpret_cast<const unsigned long long*>(src)[w % 16];
+      }
+    }
     // the previous interval of this chain may have run on another SM: thread 0 acquired its
     // release; every thread orders its loads (and, through the proxy fence, this CTA's bulk
     // copies) after it
@@ -187,19 +196,15 @@ k_sweep(const HqChain* __restrict__ chains, int nchains, const int2* __restrict_
     udt_body<2>(ch, side, b, true, smem, mv, true);
     __syncthreads();
     mark(3);
-    const HqGemmJob* const* L = lists + ((size_t)dir * nstab_max + b) * 5;
     // the push product and the equal-time G builder (src/dqmc_core.cpp:204-215 / :265-276):
-    // products PH_PUSH, B1, B2, the inverse, products B3, B4; each product's job is staged in
-    // shared memory (one call site of the GEMM)
+    // products PH_PUSH, B1, B2, the inverse, products B3, B4 (one call site of the GEMM)
     for (int ph = 0; ph < 5; ++ph) {
       if (ph == 3) {
         invert_body<2>(ch, 0, true, smem, pv);
         __syncthreads();
         mark(6);
       }
-      if (threadIdx.x == 0) job = L[ph][c];
-      __syncthreads();
-      gemm_cta(job, smem, red);
+      gemm_cta(jobs[ph], smem, red);
       if (ph == 0) mark(4);
       if (ph == 2) mark(5);
     }

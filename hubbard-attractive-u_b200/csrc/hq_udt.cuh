@@ -57,8 +57,16 @@ static __device__ void qr_panel(double* A, int ld, int N, int p0, int p1, double
   }
 }
 
-// reflector of column c (dlarfg convention) by the warp that holds the column in registers
-// (x[t] = A[lane + 32 t, c]); writes the column (R entries, beta, v) and tau[c]
+// rows of a lane's column in registers: x[t] = row lane + 32 t, t < RPL = ceil(N / 32), so that only
+// the last may lie past the matrix
+template <int RPL>
+__device__ __forceinline__ bool row_ok(int t, int r, int N) {
+  return t + 1 < RPL || r < N;
+}
+
+// Reflector of column c (dlarfg convention) by the warp that holds the column in registers; writes
+// the column (R entries, beta, v) and tau[c]. Straight code: a zero column below the diagonal (xs =
+// 0) takes tau = 0 and the factor 1 by selection.
 template <int RPL>
 __device__ __forceinline__ void reflector_reg(double* A, int ld, int N, int c, double (&x)[RPL], double* tau) {
   const int lane = threadIdx.x & 31;
@@ -67,43 +75,38 @@ __device__ __forceinline__ void reflector_reg(double* A, int ld, int N, int c, d
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
     const int r = lane + 32 * t;
-    if (r > c && r < N) {
-      if (t & 1) xs1 = fma(x[t], x[t], xs1);
-      else xs0 = fma(x[t], x[t], xs0);
-    }
-    if (r == c) alpha = x[t];
+    const double v = (r > c && row_ok<RPL>(t, r, N)) ? x[t] : 0.0;
+    if (t & 1) xs1 = fma(v, v, xs1);
+    else xs0 = fma(v, v, xs0);
+    alpha = (r == c) ? x[t] : alpha;
   }
   const double xs = warp_sum(xs0 + xs1);
   alpha = __shfl_sync(0xffffffffu, alpha, c & 31);
-  double ti = 0.0, beta = alpha;
-  if (xs > 0.0) {
-    // xs is an unscaled sum of squares already, so the norm needs no hypot
-    beta = -copysign(sqrt(fma(alpha, alpha, xs)), alpha);
-    ti = (beta - alpha) * __drcp_rn(beta);  // (beta - alpha) / beta
-    const double sc = 1.0 / (alpha - beta);
-#pragma unroll
-    for (int t = 0; t < RPL; ++t) {
-      const int r = lane + 32 * t;
-      if (r > c && r < N) x[t] *= sc;
-    }
-  }
+  const bool some = xs > 0.0;
+  // xs is an unscaled sum of squares already, so the norm needs no hypot
+  const double nb = -copysign(sqrt(fma(alpha, alpha, xs)), alpha);
+  const double beta = some ? nb : alpha;
+  const double rb = __drcp_rn(some ? nb : 1.0), rs = __drcp_rn(some ? alpha - nb : 1.0);
+  const double ti = some ? (nb - alpha) * rb : 0.0;  // (beta - alpha) / beta
+  double* Ac = A + (size_t)c * ld;
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
     const int r = lane + 32 * t;
-    if (r == c) x[t] = beta;
-    if (r < N) A[r + (size_t)c * ld] = x[t];
+    x[t] = (r == c) ? beta : (r > c ? x[t] * rs : x[t]);
+    if (row_ok<RPL>(t, r, N)) Ac[r] = x[t];
   }
-  if (lane == 0) tau[c] = ti;
+  tau[c] = ti;  // every lane the same value
 }
 
 // Householder QR of the panel columns [p0, p1) for N <= 32 RPL: the panel's kQB columns are held
 // in registers, CPW per warp by kQB / CPW warps (warp w holds columns p0 + w + i kQB / CPW);
 // the owner of column c+1 forms reflector c+1 right after applying reflector c, so one block
-// barrier separates consecutive reflectors
+// barrier separates consecutive reflectors. Bound by that chain (two warp sums, a square root and
+// two reciprocals per column). RPL = ceil(N / 32): 16 x 16 matrices took the time of five row slots.
 template <int RPL, int CPW>
 __device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* tau) {
   constexpr int NWP = kQB / CPW;  // warps that hold panel columns
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index();
   int col[CPW];
   bool own[CPW];
   double x[CPW][RPL];
@@ -114,7 +117,7 @@ __device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* t
 #pragma unroll
     for (int t = 0; t < RPL; ++t) {
       const int r = lane + 32 * t;
-      x[i][t] = (own[i] && r < N) ? A[r + (size_t)col[i] * ld] : 0.0;
+      x[i][t] = (own[i] && row_ok<RPL>(t, r, N)) ? A[r + (size_t)col[i] * ld] : 0.0;
     }
   }
   if (warp == 0) reflector_reg<RPL>(A, ld, N, p0, x[0], tau);
@@ -123,25 +126,20 @@ __device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* t
 #pragma unroll
     for (int i = 0; i < CPW; ++i) {
       if (own[i] && col[i] > c) {
-        const double ti = tau[c];
-        if (ti != 0.0) {
-          double v[RPL];
-          double w0 = 0.0, w1 = 0.0;  // two partial sums (a shorter chain per lane)
+        const double ti = tau[c];  // 0: the identity (w = 0 below)
+        double v[RPL];
+        double w0 = 0.0, w1 = 0.0;  // two partial sums (a shorter chain per lane)
 #pragma unroll
-          for (int t = 0; t < RPL; ++t) {
-            const int r = lane + 32 * t;
-            v[t] = (r > c && r < N) ? A[r + (size_t)c * ld] : 0.0;
-            if (t & 1) w1 = (r == c) ? w1 + x[i][t] : fma(v[t], x[i][t], w1);
-            else w0 = (r == c) ? w0 + x[i][t] : fma(v[t], x[i][t], w0);
-          }
-          const double w = warp_sum(w0 + w1) * ti;
-#pragma unroll
-          for (int t = 0; t < RPL; ++t) {
-            const int r = lane + 32 * t;
-            if (r == c) x[i][t] -= w;
-            else x[i][t] = fma(-w, v[t], x[i][t]);
-          }
+        for (int t = 0; t < RPL; ++t) {
+          const int r = lane + 32 * t;
+          const double vr = row_ok<RPL>(t, r, N) ? A[r + (size_t)c * ld] : 0.0;
+          v[t] = r > c ? vr : (r == c ? 1.0 : 0.0);
+          if (t & 1) w1 = fma(v[t], x[i][t], w1);
+          else w0 = fma(v[t], x[i][t], w0);
         }
+        const double w = warp_sum(w0 + w1) * ti;
+#pragma unroll
+        for (int t = 0; t < RPL; ++t) x[i][t] = fma(-w, v[t], x[i][t]);
         if (col[i] == c + 1) reflector_reg<RPL>(A, ld, N, c + 1, x[i], tau);
       }
     }
@@ -491,15 +489,20 @@ __device__ __forceinline__ void udt_body(const HqChain& ch, int side, int b, boo
   // others does not matter, as every later panel selects by norm again) ----
   for (int p0 = 0; p0 < N; p0 += kQB) {
     const int p1 = min(p0 + kQB, N);
-    if (N <= 160) {
-      panel_pivot<5>(A, ld, N, p0, p1, nrm, order, rk, Vb, ldp, mv);
+    // panel pivoting and QR with ceil(N / 32) row slots per lane
+    auto panel = [&](auto rc) {
+      constexpr int RPL = decltype(rc)::value;
+      panel_pivot<RPL>(A, ld, N, p0, p1, nrm, order, rk, Vb, ldp, mv);
       phase(1);
-      qr_panel_reg<5, CPW>(A, ld, N, p0, p1, tau);
-    } else {
-      panel_pivot<0>(A, ld, N, p0, p1, nrm, order, rk, Vb, ldp, mv);
-      phase(1);
-      qr_panel(A, ld, N, p0, p1, tau);
-    }
+      if constexpr (RPL > 0) qr_panel_reg<RPL, CPW>(A, ld, N, p0, p1, tau);
+      else qr_panel(A, ld, N, p0, p1, tau);
+    };
+    if (N <= 32) panel(IntC<1>{});
+    else if (N <= 64) panel(IntC<2>{});
+    else if (N <= 96) panel(IntC<3>{});
+    else if (N <= 128) panel(IntC<4>{});
+    else if (N <= 160) panel(IntC<5>{});
+    else panel(IntC<0>{});
     phase(2);
     if (p1 < N) {
       double* Tp = Tc + (size_t)(p0 / kQB) * kQB * kQB;

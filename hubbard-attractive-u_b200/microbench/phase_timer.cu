@@ -1,7 +1,7 @@
 // phase_timer.cu -- clock64 phase timings of the per-chain kernel bodies on one B200, for N = 144
-// (the 12 x 12 lattice): the Gauss-Jordan inverse (invert_body) and the UDV push factorisation
+// (the 12 x 12 lattice; -DHQ_TIMER_N=64, say, for another): the Gauss-Jordan inverse (invert_body) and the UDV push factorisation
 // (udt_body), run through the library's own bodies with a phase hook that synchronises the block
-// and reads the clock; the delayed-update flush of the interval kernel (flush_block) at ranks
+// and reads the clock; the delayed-update flush of the interval kernel (rank_strips) at ranks
 // 4..16; the one-CTA builder products of the persistent sweep (gemm_cta) for each job case.
 // One CTA per matrix, 128 (factorisations) or 148 (flush, products) CTAs, synthetic operands.
 // Build: make -C hubbard-attractive-u_b200/microbench; run: ./phase_timer (one GPU).
@@ -16,7 +16,10 @@
 
 using namespace hq;
 
-constexpr int kN = 144;
+#ifndef HQ_TIMER_N
+#define HQ_TIMER_N 144
+#endif
+constexpr int kN = HQ_TIMER_N;
 constexpr int kSlots = 8;
 
 // phase hook: cycles since the previous mark, per phase slot (kept by thread 0)
@@ -77,11 +80,14 @@ __global__ void __launch_bounds__(NT, 1) k_udt_phases(const double* X, double* U
 
 __global__ void __launch_bounds__(HQ_INT_THREADS, 1) k_flush(unsigned long long* clk, int k, int reps) {
   extern __shared__ __align__(16) double smem[];
-  const int ld = interval_ld(kN), ldp = panel_ld(kN);
+  const int ld = interval_ld(kN), ldp = panel_ld(pad16(kN));
   double* G = smem;
-  double* X = G + kN * ld;
+  double* X = G + resident_doubles(kN);
   double* Y = X + ldp * 16;
-  for (int i = threadIdx.x; i < kN * ld; i += blockDim.x) G[i] = 1e-3 * ((i * 37 + blockIdx.x) % 101);
+  MetroShared sh{};
+  sh.X = X;
+  sh.Y = Y;
+  for (int i = threadIdx.x; i < (int)resident_doubles(kN); i += blockDim.x) G[i] = 1e-3 * ((i * 37 + blockIdx.x) % 101);
   for (int i = threadIdx.x; i < ldp * 16; i += blockDim.x) {
     X[i] = 1e-3 * ((i * 13) % 17 - 8);
     Y[i] = 1e-3 * ((i * 7) % 19 - 9);
@@ -89,7 +95,7 @@ __global__ void __launch_bounds__(HQ_INT_THREADS, 1) k_flush(unsigned long long*
   __syncthreads();
   const long long t0 = clock64();
   for (int r = 0; r < reps; ++r) {
-    flush_block(G, ld, kN, X, ldp, Y, ldp, k);
+    for_ksteps(k, [&](auto kc) { rank_strips<pad16(kN) / 16, tile_cols(kN), decltype(kc)::value>(G, ld, sh, ldp, ldp); });
     __syncthreads();
   }
   if (threadIdx.x == 0) atomicAdd(clk, (unsigned long long)(clock64() - t0));
@@ -222,9 +228,9 @@ int main() {
 
   // the flush of one 16-site block of delayed updates at rank k
   {
-    const size_t smem = ((size_t)kN * interval_ld(kN) + 2 * panel_ld(kN) * 16) * 8;
+    const size_t smem = (resident_doubles(kN) + 2 * panel_ld(pad16(kN)) * 16) * 8;
     cudaFuncSetAttribute(k_flush, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    std::printf("flush_block (G += X Y, G 144 x 144 in shared memory, 8 warps):\n");
+    std::printf("flush (G += X Y, G N x N in shared memory, 8 warps):\n");
     for (int k : {4, 8, 10, 12, 16}) {
       const int reps = 200;
       cudaMemset(clk, 0, 8);
@@ -267,7 +273,7 @@ int main() {
                           {"B4: U_R W2, k-scaling, wrap error", 0, 0, 2, 0, 0, 1, 0.0},
                           {"(no transpose) k-scaling only", 0, 0, 2, 0, 0, 0, 0.0},
                           {"(no transpose) wrap error only", 0, 0, 0, 0, 0, 1, 0.0}};
-    std::printf("gemm_cta (one 144^3 product per CTA, 8 warps, operands from HBM):\n");
+    std::printf("gemm_cta (one N^3 product per CTA, 8 warps, operands from HBM):\n");
     for (const Case& cs : cases) {
       HqGemmJob j{};
       j.M = j.Nc = j.K = kN;
