@@ -10,6 +10,10 @@
 
 namespace hq {
 
+// a compile-time integer as an argument
+template <int V>
+struct IntC { static constexpr int value = V; };
+
 constexpr int kQB = 16;  // column panel of the blocked Householder UDV factorisation
 constexpr int kGJ = 16;  // pivot panel of the blocked Gauss-Jordan inverse
 
@@ -20,9 +24,6 @@ struct NoPhase {
   __device__ __forceinline__ void operator()(int) const {}
 };
 
-// shared-memory leading dimension of an N x N matrix: odd, so that threads walking
-// consecutive columns hit distinct banks
-__host__ __device__ constexpr inline int smem_ld(int N) { return (N % 2 == 0) ? N + 1 : N; }
 
 // leading dimension of the delayed-update panels: = 4 (mod 16) doubles, so that the DMMA
 // fragment loads of the flush are free of bank conflicts
@@ -40,6 +41,10 @@ __host__ __device__ constexpr inline int tile_cols(int N) {
 // so that the DMMA accumulator tiles of the rank updates (lane 4g+q at row g, columns 2q, 2q+1) and
 // the 16-byte accesses of lanes that walk columns are free of bank conflicts
 __host__ __device__ constexpr inline int interval_ld(int N) { return pad16(N) + 2; }
+// The factorisations and the B chain use the same leading dimension: the DMMA fragments of their
+// trailing updates are then at most two-way (four-way at an odd one; 144 x 144 inverse 293k -> 273k
+// cycles, push 413k -> 388k) and the B chain's passes move 16-byte words (178k -> 164k per interval).
+__host__ __device__ constexpr inline int smem_ld(int N) { return interval_ld(N); }
 // doubles of a resident G: columns padded to the tiles of the flush
 __host__ __device__ constexpr inline size_t resident_doubles(int N) { return (size_t)interval_ld(N) * 8 * tile_cols(N); }
 
@@ -118,16 +123,26 @@ __device__ __forceinline__ void cp_async_8(double* dst, const double* src, bool 
   const int nbytes = valid ? 8 : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(nbytes));
 }
+// 16-byte copy, both addresses 16-byte aligned
+__device__ __forceinline__ void cp_async_16(double* dst, const double* src) {
+  const unsigned saddr = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(src));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int NPEND>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(NPEND)); }
 
-// global -> shared copy of an N x N column-major matrix (shared ld `ldd`): every element is
-// an asynchronous copy, all issued before one wait, so that the copy costs about one memory
+// global -> shared copy of an N x N column-major matrix (shared ld `ldd`): every element (or
+// aligned pair) is an asynchronous copy, all issued before one wait, so that the copy costs about one memory
 // latency rather than one per loop trip. On return this thread's copies have landed; the
 // caller's barrier makes all of them visible.
 __device__ __forceinline__ void load_mat_async(double* dst, int ldd, const double* src, int lds, int N) {
-  HQ_FOR_EACH_ELEM(N, i, j) cp_async_8(dst + i + (size_t)j * ldd, src + i + (size_t)j * lds, true);
+  if (((N | ldd | lds) & 1) == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+    for (int j = (int)(threadIdx.x >> 5); j < N; j += (int)(blockDim.x >> 5))
+      for (int i = 2 * (int)(threadIdx.x & 31); i < N; i += 64) cp_async_16(dst + i + (size_t)j * ldd, src + i + (size_t)j * lds);
+  } else {
+    HQ_FOR_EACH_ELEM(N, i, j) cp_async_8(dst + i + (size_t)j * ldd, src + i + (size_t)j * lds, true);
+  }
   cp_async_commit();
   cp_async_wait<0>();
 }
@@ -216,11 +231,53 @@ __device__ __forceinline__ void store_mat_bulk(double* dst, const double* src, i
   }
 }
 
+// G[0:M, 0:Nc] += X[0:M, 0:16] Y[0:16, 0:Nc] for M a multiple of 16 and Nc of 8 (X column-major
+// ldx, Y row-major ldy), nothing checked: 16 x 24 strips, the last of a row of strips narrower
+static __device__ void rank16_update(double* G, int ld, int M, int Nc, const double* X, int ldx, const double* Y, int ldy) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, q = lane & 3;
+  const int mt = M / 16, tc = Nc / 8, ns = (tc + 2) / 3;
+  for (int st = warp; st < mt * ns; st += nw) {
+    const int sc = st / mt, r0 = (st - sc * mt) * 16, t0 = 3 * sc;
+    double* Gp = G + r0 + g + (size_t)(8 * t0 + 2 * q) * ld;
+    const double* Xp = X + r0 + g + q * ldx;
+    const double* Yp = Y + q * ldy + 8 * t0 + g;
+    auto strip = [&](auto nc) {
+      constexpr int NT = decltype(nc)::value;
+      double acc[NT][4];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        acc[t][0] = Gp[(size_t)(8 * t) * ld];
+        acc[t][1] = Gp[(size_t)(8 * t + 1) * ld];
+        acc[t][2] = Gp[8 + (size_t)(8 * t) * ld];
+        acc[t][3] = Gp[8 + (size_t)(8 * t + 1) * ld];
+      }
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const double a0 = Xp[4 * s * ldx], a1 = Xp[8 + 4 * s * ldx];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) dmma_16x8x4(acc[t], a0, a1, Yp[4 * s * ldy + 8 * t]);
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        Gp[(size_t)(8 * t) * ld] = acc[t][0];
+        Gp[(size_t)(8 * t + 1) * ld] = acc[t][1];
+        Gp[8 + (size_t)(8 * t) * ld] = acc[t][2];
+        Gp[8 + (size_t)(8 * t + 1) * ld] = acc[t][3];
+      }
+    };
+    if (tc - t0 >= 3) strip(IntC<3>{});
+    else if (tc - t0 == 2) strip(IntC<2>{});
+    else strip(IntC<1>{});
+  }
+}
+
 // G[0:M, 0:Nc] += X[0:M, 0:k] Y[0:k, 0:Nc]  (X column-major ldx, Y row-major ldy, k <= 16),
 // by 16 x 32 strips of four 16 x 8 DMMA tiles that share the A fragments; the fragments of
 // all k-steps are loaded before the strip's G tiles so that their latencies overlap
 static __device__ void rank_update(double* G, int ld, int M, int Nc, const double* X, int ldx, const double* Y, int ldy,
                             int k) {
+  if (k == 16 && M % 16 == 0 && Nc % 8 == 0) return rank16_update(G, ld, M, Nc, X, ldx, Y, ldy);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, q = lane & 3;
   const int mt = (M + 15) / 16, ns = (Nc + 31) / 32;
@@ -297,15 +354,15 @@ __device__ __forceinline__ void scale_cols(double* M, int ld, int N, const doubl
 }
 
 // M <- e^{V} expK M (AFTER true) or expK e^{V} M (AFTER false), v = e^{V}, by the dense or the
-// separable form. RES: M in shared memory with the leading dimension ldr(N) (a compile-time value
-// per lattice size); otherwise any leading dimension. Ends with a barrier.
+// separable form. RES: M in shared memory with the leading dimension interval_ld(N) (a compile-time
+// value per lattice size); otherwise any leading dimension. Ends with a barrier.
 enum SideOp { LEFT_B, LEFT_BT, RIGHT_BINV };  // e^V E M,  E e^V M,  M E^-1 e^-V
-template <int OP, bool RES, int PAD>
+template <int OP, bool RES>
 __device__ __forceinline__ void apply_side(const HqChain& ch, double* M, int ld, const double* v, double* stage) {
   if (ch.expk_mode == HQK_EXPK_SEPARABLE) {
     for_lattice(ch.L, [&](auto lc) {
       constexpr int L = decltype(lc)::value, N = L * L;
-      constexpr int LD = !RES || L > 12 ? 0 : (PAD ? interval_ld(N) : smem_ld(N));
+      constexpr int LD = !RES || L > 12 ? 0 : interval_ld(N);
       if constexpr (OP == LEFT_B) sep_one<L, LD, 0, 2>(M, ld, ch.sep_a, ch.sep_c, v);
       else if constexpr (OP == LEFT_BT) sep_one<L, LD, 0, 1>(M, ld, ch.sep_a, ch.sep_c, v);
       else sep_one<L, LD, 1, 2>(M, ld, ch.sep_ai, ch.sep_ci, v);

@@ -75,12 +75,14 @@ inline double canonical(uint32_t& x) {
 //  exp(dt t H_1d) is circulant with a[d] = (1/L) sum_k exp(2 dt t cos(2 pi k/L)) cos(2 pi k d/L).
 // ---------------------------------------------------------------------------------------
 void circulant_exp(int L, double dt_t, double* a) {
+  long double th[32], ek[32];  // L <= 32: N <= HQ_MAX_N = 1024
+  for (int k = 0; k < L; ++k) {
+    th[k] = 2.0L * 3.14159265358979323846264338327950288L * k / L;
+    ek[k] = std::exp(2.0L * dt_t * std::cos(th[k]));
+  }
   for (int d = 0; d < L; ++d) {
     long double acc = 0.0L;
-    for (int k = 0; k < L; ++k) {
-      const long double th = 2.0L * 3.14159265358979323846264338327950288L * k / L;
-      acc += std::exp(2.0L * dt_t * std::cos(th)) * std::cos(th * d);
-    }
+    for (int k = 0; k < L; ++k) acc += ek[k] * std::cos(th[k] * d);
     a[d] = static_cast<double>(acc / L);
   }
 }
@@ -192,7 +194,7 @@ struct hq_ctx {
   char* arena = nullptr;
   size_t arena_bytes = 0;
   std::vector<void*> extra_allocs;
-  int Nmax = 0, kmax_max = 0, ntmax = 0, nstab_max = 0;
+  int Nmax = 0, kmax_max = 0, ntmax = 0, nstab_max = 0, pace_max = 0;
   bool resident = true;         // matrices fit in one SM's shared memory
   bool cluster_interval = false;  // the interval kernel may run on four-CTA clusters (16 x 16 lattices)
   bool cluster_capable = false;   // the device can run them (the autotuner may switch them off)
@@ -719,9 +721,8 @@ void issue_sweep(hq_ctx* c, int dir, int flags) {
       builder_inverse(c, 3, b, true);
       run_jobs(c, {PH_B3, PH_D4}, 3, b);         // W2 = Y = T1^-1 dlmax^-1 U_L^T, W5 = T1^-1 dlmin Vt_L
       run_jobs(c, {PH_D3, PH_D5, PH_D6}, 3, b);  // W3 = G(t,t), W0 = G(t,0), W4 = G(0,t)
-      { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_commit(c->d_desc, c->n, b, c->stream)); }
-      { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_store(c->d_desc, c->n, b, c->stream)); }
-      { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_measure(c->d_desc, c->n, b, 0, c->stream)); }
+      { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_commit(c->d_desc, c->n, b, c->Nmax, c->stream)); }
+      { ProfScope ps(c, PC_DYN); HQ_CUDA(hq::launch_dyn_measure(c->d_desc, c->n, b, c->pace_max, c->stream)); }
     }
   }
 }
@@ -788,6 +789,7 @@ int hq_create(int device, int n_chains, const hq_chain_params* params, hq_ctx** 
     if (p.nl > HQ_MAX_L) h.expk_mode = HQ_EXPK_DENSE;
     c->Nmax = std::max(c->Nmax, h.N);
     c->ntmax = std::max(c->ntmax, p.nt);
+    c->pace_max = std::max(c->pace_max, std::min(p.nt, p.stabilization_pace));
     c->nstab_max = std::max(c->nstab_max, h.n_stab);
     if (p.dynamic) c->has_dynamic = true;
   }
@@ -986,6 +988,14 @@ int hq_create(int device, int n_chains, const hq_chain_params* params, hq_ctx** 
   build_jobs(c.get());
   if (c->resident && hq::sweep_fits(c->Nmax, c->kmax_max, optin)) {
     setup_sweep(c.get());
+    // Small chains run persistently unless told otherwise: an interval takes them less time than the
+    // launches and the gaps between them. One round trip of 40 slices, launches / persistent, ms: 64
+    // chains of 4x4 1.36 / 0.99, 6x6 2.59 / 2.14, 8x8 3.27 / 3.03, 9x9 5.20 / 5.66, 12x12 10.8 / 12.1;
+    // 256 chains of 6x6 4.19 / 4.15, 8x8 5.51 / 5.74. Larger chains gain more from the launch
+    // sequence's 16-warp factorisations and products over several SMs, and so do those of 7x7 and
+    // 8x8 once there are more of them than SMs.
+    if (c->sweep_capable && (c->Nmax <= 36 || (c->Nmax <= 64 && c->n <= c->sweep_grid)))
+      c->sweep_mode = HQ_SWEEP_PERSISTENT;
     // HQ_SWEEP_MODE=persistent | launches overrides the default mode (for comparisons)
     const char* m = std::getenv("HQ_SWEEP_MODE");
     if (m && std::strcmp(m, "persistent") == 0) c->sweep_mode = HQ_SWEEP_PERSISTENT;
@@ -1667,9 +1677,8 @@ int hq_logdet_adjoint(hq_ctx* c, double* out, double* logdet) {
 //  that must never meet an out-of-memory failure in the middle of its work. For them,
 //  hq_equaltime_g_noalloc computes the equal-time Green's function
 //  G(0,0) = (1 + B(nt-1)...B(0))^-1 of one chain from Ising fields already on the device,
-//  with every temporary (the UDV stack, the work matrices, the chain descriptor and the GEMM
-//  job lists) held in one file-scope device array of fixed size. The work is the kernel
-//  sequence of hq_init_stacks_and_g.
+//  with every temporary (the UDV stack and the work matrices) held in one file-scope device array
+//  of fixed size. The work is that of hq_init_stacks_and_g in one launch (k_equaltime).
 // =======================================================================================
 namespace {
 
@@ -1691,11 +1700,7 @@ int set_error(int code, const std::string& msg) {
   return code;
 }
 
-// exp(dt t H_1d) of the L-site periodic chain is circulant:
-// a[d] = (1/L) sum_k exp(2 dt t cos(2 pi k / L)) cos(2 pi k d / L)
-void circulant(int L, double dt_t, double* a) { circulant_exp(L, dt_t, a); }
 size_t up256(size_t b) { return align256(b); }
-HqGemmJob job(int N, const double* A, int ta, const double* B, int tb, double* C) { return make_job(N, A, ta, B, tb, C); }
 
 }  // namespace
 
@@ -1738,122 +1743,40 @@ static int equaltime_g_noalloc(int nl, double nnt, double u, double mu, double b
   const size_t NN = size_t(N) * N, mat = NN * sizeof(double);
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += up256(bytes); return o; };
-  const size_t o_desc = take(sizeof(HqChain));
-  const int njobs = n_stab + 4;
-  const size_t o_jobs = take(sizeof(HqGemmJob) * njobs);
   const size_t o_U = take(2 * size_t(n_stab) * mat);
   const size_t o_D = take(2 * size_t(n_stab) * N * sizeof(double));
   const size_t o_Vt = take(2 * size_t(n_stab) * mat);
-  const size_t o_X = take(mat);
-  size_t o_W[4];
+  size_t o_W[2];
   for (auto& w : o_W) w = take(mat);
-  const size_t o_I = take(mat);
-  const size_t o_one = take(N * sizeof(double));
-  const size_t o_E = take(2 * mat);
   const size_t o_acc = take(HQ_ACC_COUNT * sizeof(double));
-  const size_t o_rng = take(sizeof(uint32_t));
   if (off > kScratchBytes) return set_error(HQ_E_RANGE, "hq_equaltime_g_noalloc: scratch layout exceeds 4 MiB");
   auto ptr = [&](size_t o) { return reinterpret_cast<double*>(base + o); };
 
-  // ---- model constants (src/hubbard.cpp:25-49) ----
+  // ---- model constants (src/hubbard.cpp:25-49); N <= 64: the separable exp(-dt K) ----
   const double dt = beta / nt;
   const double alpha = std::acosh(std::exp(0.5 * dt * u));
   HqChain d;
   std::memset(&d, 0, sizeof(d));
   d.N = N; d.L = nl; d.nt = nt; d.pace = pace; d.n_stab = n_stab;
-  d.expk_mode = (nl <= HQ_MAX_L) ? HQK_EXPK_SEPARABLE : HQK_EXPK_DENSE;
+  d.expk_mode = HQK_EXPK_SEPARABLE;
   d.kmax = 4; d.active = 1;
   d.alpha = alpha; d.dt = dt;
-  d.delta_p = std::exp(-2 * alpha) - 1;
-  d.delta_m = std::exp(2 * alpha) - 1;
   d.ev_p = std::exp(alpha);
   d.ev_m = std::exp(-alpha);
   d.sep_c = std::exp(dt * mu);
   d.sep_ci = std::exp(-dt * mu);
-  circulant(nl, dt * nnt, d.sep_a);
-  circulant(nl, -dt * nnt, d.sep_ai);
-  d.expK = ptr(o_E);
-  d.inv_expK = ptr(o_E) + NN;
+  circulant_exp(nl, dt * nnt, d.sep_a);
   d.G = g_dev;
   d.fields = reinterpret_cast<int8_t*>(const_cast<signed char*>(fields_dev));
-  d.rng = reinterpret_cast<uint32_t*>(base + o_rng);
-  d.X = ptr(o_X);
   d.stackU = ptr(o_U);
   d.stackD = ptr(o_D);
   d.stackVt = ptr(o_Vt);
-  d.W0 = ptr(o_W[0]); d.W1 = ptr(o_W[1]); d.W2 = ptr(o_W[2]); d.W3 = ptr(o_W[3]);
-  d.W4 = d.W3; d.W5 = d.W3;  // not used by this sequence
+  d.W0 = ptr(o_W[0]);
+  d.W1 = ptr(o_W[1]);
   d.acc = ptr(o_acc);
-
-  // host images of the constant inputs: dense expK, identity, ones (copied on the caller's
-  // stream; pageable sources are consumed before cudaMemcpyAsync returns)
-  std::vector<double> a(nl), ai(nl), E(2 * NN), I(NN, 0.0), one(N, 1.0);
-  circulant(nl, dt * nnt, a.data());
-  circulant(nl, -dt * nnt, ai.data());
-  for (int j = 0; j < N; ++j)
-    for (int i = 0; i < N; ++i) {
-      const int dx = ((i % nl) - (j % nl) + nl) % nl, dy = ((i / nl) - (j / nl) + nl) % nl;
-      E[i + size_t(j) * N] = d.sep_c * a[dx] * a[dy];
-      E[NN + i + size_t(j) * N] = d.sep_ci * ai[dx] * ai[dy];
-    }
-  for (int k = 0; k < N; ++k) I[k + size_t(k) * N] = 1.0;
-
-  // ---- batched GEMM jobs: stack pushes, then the builder with an empty left stack ----
-  std::vector<HqGemmJob> jobs;
-  const double* Iid = ptr(o_I);
-  const double* ones = ptr(o_one);
-  for (int b = 0; b < n_stab; ++b) {
-    const double* prev = (b == 0) ? Iid : d.stackVt + (size_t(n_stab) + (b - 1)) * NN;
-    jobs.push_back(job(N, d.W0, 0, prev, 0, d.stackVt + (size_t(n_stab) + b) * NN));
-  }
-  const double* UR = d.stackU + (size_t(n_stab) + n_stab - 1) * NN;
-  const double* DR = d.stackD + (size_t(n_stab) + n_stab - 1) * N;
-  const double* VtR = d.stackVt + (size_t(n_stab) + n_stab - 1) * NN;
-  HqGemmJob b1 = job(N, Iid, 1, UR, 0, d.W1);
-  b1.rs = ones; b1.rs_mode = 2; b1.cs = DR; b1.cs_mode = 2;
-  HqGemmJob b2 = job(N, Iid, 0, VtR, 1, d.W1);
-  b2.rs = ones; b2.rs_mode = 3; b2.cs = DR; b2.cs_mode = 3; b2.beta = 1.0;
-  HqGemmJob b3 = job(N, d.W1, 0, Iid, 1, d.W2);
-  b3.ks = ones; b3.ks_mode = 2;
-  HqGemmJob b4 = job(N, UR, 0, d.W2, 0, g_dev);
-  b4.ks = DR; b4.ks_mode = 2;
-  jobs.push_back(b1);
-  jobs.push_back(b2);
-  jobs.push_back(b3);
-  jobs.push_back(b4);
-
-  // ---- upload (no allocation) and launch ----
-  cudaError_t e = cudaSuccess;
-  HqChain* d_desc = reinterpret_cast<HqChain*>(base + o_desc);
-  HqGemmJob* d_jobs = reinterpret_cast<HqGemmJob*>(base + o_jobs);
-  if ((e = cudaMemcpyAsync(d_desc, &d, sizeof(d), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(d_jobs, jobs.data(), jobs.size() * sizeof(HqGemmJob), cudaMemcpyHostToDevice, st)) !=
-          cudaSuccess ||
-      (e = cudaMemcpyAsync(ptr(o_E), E.data(), E.size() * sizeof(double), cudaMemcpyHostToDevice, st)) !=
-          cudaSuccess ||
-      (e = cudaMemcpyAsync(ptr(o_I), I.data(), I.size() * sizeof(double), cudaMemcpyHostToDevice, st)) !=
-          cudaSuccess ||
-      (e = cudaMemcpyAsync(ptr(o_one), one.data(), one.size() * sizeof(double), cudaMemcpyHostToDevice, st)) !=
-          cudaSuccess ||
-      (e = cudaMemsetAsync(ptr(o_acc), 0, HQ_ACC_COUNT * sizeof(double), st)) != cudaSuccess)
-    return set_error(HQ_E_CUDA, std::string("hq_equaltime_g_noalloc: upload: ") + cudaGetErrorString(e));
-  // the kernels' shared-memory limits (raised only, and only when an earlier context of
-  // smaller chains left them below this size; no allocation)
-  if ((e = hq::prepare_kernels(N, 4, true)) != cudaSuccess)
-    return set_error(HQ_E_CUDA, std::string("hq_equaltime_g_noalloc: kernel limits: ") + cudaGetErrorString(e));
-  for (int b = 0; b < n_stab && e == cudaSuccess; ++b) {
-    // src/dqmc_core.cpp:67-87: B^T products from t = nt down to 1, pushed every pace slices
-    e = hq::launch_bchain(d_desc, 1, HQ_DOWN, b, N, true, st);
-    if (e == cudaSuccess) e = hq::launch_udt(d_desc, 1, 1, b, N, true, st);
-    if (e == cudaSuccess) e = hq::launch_gemm(d_jobs + b, 1, N, N, st);
-  }
-  // src/dqmc_core.cpp:89-97 with stable_numerics.hpp:186-239: G = (1 + right^T)^-1
-  const int jb = n_stab;
-  if (e == cudaSuccess) e = hq::launch_gemm(d_jobs + jb, 1, N, N, st);
-  if (e == cudaSuccess) e = hq::launch_gemm(d_jobs + jb + 1, 1, N, N, st);
-  if (e == cudaSuccess) e = hq::launch_invert(d_desc, 1, n_stab - 1, 0, N, true, st);
-  if (e == cudaSuccess) e = hq::launch_gemm(d_jobs + jb + 2, 1, N, N, st);
-  if (e == cudaSuccess) e = hq::launch_gemm(d_jobs + jb + 3, 1, N, N, st);
+  // one launch: the chain's description travels as the kernel's argument (its first launch on a
+  // device raises the kernel's shared-memory limit; no allocation)
+  const cudaError_t e = hq::launch_equaltime(d, st);
   if (e != cudaSuccess) return set_error(HQ_E_CUDA, std::string("hq_equaltime_g_noalloc: launch: ") + cudaGetErrorString(e));
   return HQ_OK;
 }

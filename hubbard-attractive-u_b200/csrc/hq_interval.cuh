@@ -100,14 +100,15 @@ __device__ __forceinline__ int metropolis_dispatch(const HqChain& ch, uint32_t r
 // of the bulk load of G (initialised for one arrival).
 struct IntervalScratch {
   double* red;     // 96 doubles
+  double* est;     // 4 doubles: the chain's estimator sums while its slices are worked on
   uint64_t* gbar;
 };
-constexpr int kIntervalScratchBytes = (96 + 2) * 8;
+constexpr int kIntervalScratchBytes = (96 + 4 + 2) * 8;
 
 // Places the interval scratch at `p` (16-byte aligned, kIntervalScratchBytes long).
 __device__ __forceinline__ IntervalScratch interval_scratch_at(void* p) {
   double* d = reinterpret_cast<double*>(p);
-  return {d, reinterpret_cast<uint64_t*>(d + 96)};
+  return {d, d + 96, reinterpret_cast<uint64_t*>(d + 100)};
 }
 
 // The update (or no-update) slices of stabilisation interval b of chain `ch` in direction dir.
@@ -139,6 +140,10 @@ __device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b,
   uint32_t rng = *ch.rng;
   double n_acc = 0.0, n_prop = 0.0;
   long long log_base = (flags & HQ_F_LOG_RATIOS) && ch.ratio_count ? *ch.ratio_count : 0;
+  // the estimator sums stay in shared memory for the interval: a round trip to global memory per
+  // slice is longer than a small lattice's passes
+  static_assert(HQ_ACC_FILLING == 0 && HQ_ACC_DOCC == 1 && HQ_ACC_SWAVE == 2 && HQ_ACC_NSLICE == 3, "the first four");
+  if (threadIdx.x < 4) sc.est[threadIdx.x] = ch.acc[threadIdx.x];
   __syncthreads();
 
   const int nsl = t_hi - t_lo + 1;
@@ -147,15 +152,23 @@ __device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b,
   // measured after stabilisation
   const bool fused = (flags & HQ_F_MEASURE) && ch.expk_mode == HQK_EXPK_SEPARABLE && wrap_measures<RES>(ch.L) &&
                      (dir == HQ_UP || dir == HQ_DOWN);
+  // the next slice's fields are on their way while a slice is worked on
+  auto field = [&](int step) {
+    const int l = ((dir == HQ_DOWN) ? (t_hi - step) : (t_lo + step)) % ch.nt;
+    return step < nsl && (int)threadIdx.x < N ? ch.fields[(size_t)l * N + threadIdx.x] : (int8_t)0;
+  };
+  int8_t next = field(0);
   for (int step = 0; step < nsl; ++step) {
     const int t = (dir == HQ_DOWN) ? (t_hi - step) : (t_lo + step);
     const int l = t % ch.nt;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) sh.s[i] = ch.fields[(size_t)l * N + i];
+    if ((int)threadIdx.x < N) sh.s[threadIdx.x] = next;
+    for (int i = threadIdx.x + blockDim.x; i < N; i += blockDim.x) sh.s[i] = ch.fields[(size_t)l * N + i];
+    next = field(step + 1);
     __syncthreads();
     if (dir != HQ_DOWN) {
       slice_factors(ch, sh.s, vp, vm);
       __syncthreads();
-      wrap_slice<RES>(ch, G, ld, vp, vm, HQ_UP, work, (fused && step > 0) ? ch.acc : nullptr, sc.red);
+      wrap_slice<RES>(ch, G, ld, vp, vm, HQ_UP, work, (fused && step > 0) ? sc.est : nullptr, sc.red);
     }
     if (dir == HQ_UP || dir == HQ_DOWN) {
       n_acc += metropolis_dispatch<RES>(ch, rng, flags, log_base);
@@ -166,12 +179,12 @@ __device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b,
     if (dir == HQ_DOWN) {
       slice_factors(ch, sh.s, vp, vm);
       __syncthreads();
-      wrap_slice<RES>(ch, G, ld, vp, vm, HQ_DOWN, work, (fused && step < nsl - 1) ? ch.acc : nullptr, sc.red);
+      wrap_slice<RES>(ch, G, ld, vp, vm, HQ_DOWN, work, (fused && step < nsl - 1) ? sc.est : nullptr, sc.red);
     }
     for (int i = threadIdx.x; i < N; i += blockDim.x) ch.fields[(size_t)l * N + i] = sh.s[i];
     if (step < nsl - 1) {
       const int lm = (dir == HQ_DOWN) ? ((t - 1) % ch.nt) : l;
-      if ((flags & HQ_F_MEASURE) && !fused) measure_slice(G, ld, N, ch.acc, sc.red);
+      if ((flags & HQ_F_MEASURE) && !fused) measure_slice(G, ld, N, sc.est, sc.red);
       if ((flags & HQ_F_SNAPSHOT) && ch.snap_tt) copy_mat(ch.snap_tt + (size_t)lm * N * N, N, G, ld, N);
     }
     __syncthreads();
@@ -181,6 +194,7 @@ __device__ __forceinline__ void interval_body(const HqChain& ch, int dir, int b,
     else copy_mat(ch.G, N, G, ld, N);
   }
   if (threadIdx.x == 0) {
+    for (int k = 0; k < 4; ++k) ch.acc[k] = sc.est[k];
     *ch.rng = rng;
     ch.acc[HQ_ACC_PROPOSED] += n_prop;
     ch.acc[HQ_ACC_ACCEPTED] += n_acc;

@@ -187,6 +187,9 @@ __device__ __forceinline__ void invert_body(const HqChain& ch, int which, bool r
     else if (N <= 96) gj_panel_reg<3, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
     else if (N <= 128) gj_panel_reg<4, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
     else if (N <= 160) gj_panel_reg<5, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (CPW == 1 && N <= 192) gj_panel_reg<CPW == 1 ? 6 : 1, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (CPW == 1 && N <= 224) gj_panel_reg<CPW == 1 ? 7 : 1, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
+    else if (CPW == 1 && N <= 256) gj_panel_reg<CPW == 1 ? 8 : 1, CPW>(A, ld, N, p0, nb, perm, fcol, pv, status);
     else for (int q = 0; q < nb; ++q) {
       const int k = p0 + q;
       if (warp == 0) {

@@ -11,6 +11,8 @@
 //  k_dyn_*     : time-displaced propagation and estimators (src/dqmc_core.cpp:291-390,
 //                include/observable_methods.hpp:84-195).
 //  k_adj_*     : adjoint of log|det(1 + B...B)| (no counterpart in the reference).
+#include <algorithm>
+
 #include "hq_phases.cuh"
 
 namespace hq {
@@ -28,13 +30,12 @@ __global__ void __launch_bounds__(HQ_INT_THREADS, 1)
 k_bchain(const HqChain* __restrict__ chains, int nchains, int dir, int b, int resident) {
   extern __shared__ __align__(16) double smem[];
   __shared__ HqChain ch;
-  __shared__ int8_t s[HQ_MAX_N];
   const int c = blockIdx.x;
   if (c >= nchains) return;
   if (threadIdx.x == 0) ch = chains[c];
   __syncthreads();
   if (!ch.active || b >= ch.n_stab) return;
-  bchain_body(ch, dir, b, resident != 0, smem, s);
+  bchain_body(ch, dir, b, resident != 0, smem);
 }
 
 // ---------------------------------------------------------------------------------
@@ -63,15 +64,14 @@ k_measure(const HqChain* __restrict__ chains, int nchains, int dir, int b, int f
 template <bool RES>
 __device__ __forceinline__ void dyn_step(const HqChain& ch, double* M, int ld, int which, const double* vp, const double* vm,
                                          double* stage) {
-  if (which != 2) apply_side<LEFT_B, RES, 1>(ch, M, ld, vp, stage);      // left multiplication by B(l) = e^V E
-  if (which != 1) apply_side<RIGHT_BINV, RES, 1>(ch, M, ld, vm, stage);  // right multiplication by B(l)^-1
+  if (which != 2) apply_side<LEFT_B, RES>(ch, M, ld, vp, stage);      // left multiplication by B(l) = e^V E
+  if (which != 1) apply_side<RIGHT_BINV, RES>(ch, M, ld, vm, stage);  // right multiplication by B(l)^-1
 }
 
 __global__ void __launch_bounds__(HQ_INT_THREADS, 1)
 k_dyn_slices(const HqChain* __restrict__ chains, int nchains, int b, int flags, int resident) {
   extern __shared__ __align__(16) double smem[];
   __shared__ HqChain ch;
-  __shared__ int8_t s[HQ_MAX_N];
   const int c = blockIdx.x, which = blockIdx.y;
   if (c >= nchains) return;
   if (threadIdx.x == 0) ch = chains[c];
@@ -92,12 +92,20 @@ k_dyn_slices(const HqChain* __restrict__ chains, int nchains, int b, int flags, 
   double* vm = vp + N;
   __syncthreads();
   const int nsl = t_hi - t_lo + 1;
+  // the next slice's fields are on their way while a slice is worked on
+  auto field = [&](int t) {
+    return t <= t_hi && (int)threadIdx.x < N ? ch.fields[(size_t)(t % ch.nt) * N + threadIdx.x] : (int8_t)0;
+  };
+  int8_t next = field(t_lo);
   for (int step = 0; step < nsl; ++step) {
     const int t = t_lo + step;
     const int l = t % ch.nt;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) s[i] = ch.fields[(size_t)l * N + i];
-    __syncthreads();
-    slice_factors(ch, s, vp, vm);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+      const bool pos = (i == (int)threadIdx.x ? next : ch.fields[(size_t)l * N + i]) > 0;
+      vp[i] = pos ? ch.ev_p : ch.ev_m;
+      vm[i] = pos ? ch.ev_m : ch.ev_p;
+    }
+    next = field(t + 1);
     __syncthreads();
     if (resident) dyn_step<true>(ch, M, ld, which, vp, vm, stage);
     else dyn_step<false>(ch, M, ld, which, vp, vm, stage);
@@ -154,9 +162,10 @@ __device__ void dyn_measure(const HqChain& ch, const double* Gt0, const double* 
 }
 
 // measure the dynamic estimators of every slice of interval b from the snapshots
-// (slices of the interval other than the last) or from the fresh G's (the last one).
+// (slices of the interval other than the last) or from the fresh G's (the last one): one CTA per
+// slice (blockIdx.y), whose sums are its own
 __global__ void __launch_bounds__(HQ_THREADS)
-k_dyn_measure(const HqChain* __restrict__ chains, int nchains, int b, int last_only) {
+k_dyn_measure(const HqChain* __restrict__ chains, int nchains, int b) {
   __shared__ HqChain ch;
   __shared__ double red[32];
   const int c = blockIdx.x;
@@ -168,7 +177,7 @@ k_dyn_measure(const HqChain* __restrict__ chains, int nchains, int b, int last_o
   int t_lo, t_hi;
   interval_range(ch.nt, ch.pace, ch.n_stab, HQ_UP, b, t_lo, t_hi);
   const size_t NN = (size_t)N * N;
-  for (int t = last_only ? t_hi : t_lo; t <= t_hi; ++t) {
+  for (int t = t_lo + (int)blockIdx.y; t <= t_hi; t += (int)gridDim.y) {
     const int l = t % ch.nt;
     const double* gt0;
     const double* g0t;
@@ -179,56 +188,45 @@ k_dyn_measure(const HqChain* __restrict__ chains, int nchains, int b, int last_o
   }
 }
 
-// at a dynamic boundary: copy the fresh G's into the snapshots of the boundary slice
-// with the tau = 0 convention (src/dqmc_core.cpp:379-387)
-__global__ void k_dyn_store(const HqChain* __restrict__ chains, int nchains, int b) {
-  const int c = blockIdx.x;
-  if (c >= nchains) return;
-  const HqChain& ch = chains[c];
-  if (!ch.active || b >= ch.n_stab) return;
-  const int N = ch.N;
-  int t_lo, t_hi;
-  interval_range(ch.nt, ch.pace, ch.n_stab, HQ_UP, b, t_lo, t_hi);
-  const int l = t_hi % ch.nt;
-  const size_t NN = (size_t)N * N;
-  for (int idx = threadIdx.x; idx < N * N; idx += blockDim.x) {
-    const int i = idx % N, j = idx / N;
-    const double gtt = ch.G[idx];
-    if (ch.snap_tt) ch.snap_tt[l * NN + idx] = gtt;
-    if (l == 0) {
-      // at tau = beta the stored pair is G(0,0), G(0,0) - 1; the propagated matrices
-      // are replaced likewise
-      ch.Gt0[idx] = gtt;
-      ch.G0t[idx] = gtt - (i == j ? 1.0 : 0.0);
-    }
-    if (ch.snap_t0) ch.snap_t0[l * NN + idx] = ch.Gt0[idx];
-    if (ch.snap_0t) ch.snap_0t[l * NN + idx] = ch.G0t[idx];
-  }
-}
-
-// commit the freshly built G(t,t), G(t,0), G(0,t) (in W3, W0, W5) after recording the
-// signed wrap errors (src/dqmc_core.cpp:334-344)
+// at a dynamic boundary: commit the freshly built G(t,t), G(t,0), G(0,t) (in W3, W0, W4) after
+// recording the signed wrap errors (src/dqmc_core.cpp:334-344), and store them into the snapshots of
+// the boundary slice with the tau = 0 convention (src/dqmc_core.cpp:379-387). A chain's elements are
+// spread over gridDim.y CTAs.
 __global__ void __launch_bounds__(HQ_THREADS) k_dyn_commit(const HqChain* __restrict__ chains, int nchains, int b) {
   __shared__ double red[32];
   const int c = blockIdx.x;
   if (c >= nchains) return;
   const HqChain& ch = chains[c];
   if (!ch.active || b >= ch.n_stab) return;
-  const int NN = ch.N * ch.N;
+  const int N = ch.N, NN = N * N;
+  int t_lo, t_hi;
+  interval_range(ch.nt, ch.pace, ch.n_stab, HQ_UP, b, t_lo, t_hi);
+  const int l = t_hi % ch.nt;
+  const size_t at = (size_t)l * NN;
   double ett = -INFINITY, edyn = -INFINITY;
-  for (int idx = threadIdx.x; idx < NN; idx += blockDim.x) {
-    const double ftt = ch.W3[idx], ft0 = ch.W0[idx], f0t = ch.W4[idx];
+  for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < NN; idx += gridDim.y * blockDim.x) {
+    const double ftt = ch.W3[idx];
+    double ft0 = ch.W0[idx], f0t = ch.W4[idx];
     ett = fmax(ett, ftt - ch.G[idx]);
     edyn = fmax(edyn, fmax(ft0 - ch.Gt0[idx], f0t - ch.G0t[idx]));
+    if (l == 0) {
+      // at tau = beta the stored pair is G(0,0), G(0,0) - 1; the propagated matrices
+      // are replaced likewise
+      ft0 = ftt;
+      f0t = ftt - (idx % N == idx / N ? 1.0 : 0.0);
+    }
     ch.G[idx] = ftt;
     ch.Gt0[idx] = ft0;
     ch.G0t[idx] = f0t;
+    if (ch.snap_tt) ch.snap_tt[at + idx] = ftt;
+    if (ch.snap_t0) ch.snap_t0[at + idx] = ft0;
+    if (ch.snap_0t) ch.snap_0t[at + idx] = f0t;
   }
   ett = block_max(ett, red);
   edyn = block_max(edyn, red);
   if (threadIdx.x == 0) {
-    ch.acc[HQ_ACC_WRAP_TT] = fmax(ch.acc[HQ_ACC_WRAP_TT], ett);
-    ch.acc[HQ_ACC_WRAP_DYN] = fmax(ch.acc[HQ_ACC_WRAP_DYN], edyn);
+    atomic_max_double(ch.acc + HQ_ACC_WRAP_TT, ett);
+    atomic_max_double(ch.acc + HQ_ACC_WRAP_DYN, edyn);
   }
 }
 
@@ -435,7 +433,7 @@ size_t smem_interval_bytes(int Nmax, int kmax, bool resident) {
   return interval_smem_doubles(Nmax, kmax, resident) * sizeof(double);
 }
 size_t smem_udt_bytes(int Nmax, bool resident) {
-  return smem_matrix_bytes(Nmax, resident, 2 * kQB * panel_ld(Nmax) + 2 * kQB * kQB + 3 * Nmax + 64 +
+  return smem_matrix_bytes(Nmax, resident, 2 * kQB * panel_ld(Nmax) + 2 * kQB * kQB + 3 * Nmax +
                                                ((Nmax - 1) / kQB) * kQB * kQB);
 }
 size_t smem_invert_bytes(int Nmax, bool resident) {
@@ -535,12 +533,8 @@ cudaError_t launch_dyn_slices(const HqChain* chains, int n, int b, int flags, in
   k_dyn_slices<<<grid, HQ_INT_THREADS, bytes, st>>>(chains, n, b, flags, resident ? 1 : 0);
   return cudaGetLastError();
 }
-cudaError_t launch_dyn_measure(const HqChain* chains, int n, int b, int last_only, cudaStream_t st) {
-  k_dyn_measure<<<n, HQ_THREADS, 0, st>>>(chains, n, b, last_only);
-  return cudaGetLastError();
-}
-cudaError_t launch_dyn_store(const HqChain* chains, int n, int b, cudaStream_t st) {
-  k_dyn_store<<<n, 256, 0, st>>>(chains, n, b);
+cudaError_t launch_dyn_measure(const HqChain* chains, int n, int b, int pace, cudaStream_t st) {
+  k_dyn_measure<<<dim3(n, std::min(pace, 32)), HQ_THREADS, 0, st>>>(chains, n, b);
   return cudaGetLastError();
 }
 cudaError_t launch_adj_interval(const HqChain* chains, int n, int b, int Nmax, bool resident, cudaStream_t st) {
@@ -568,8 +562,9 @@ cudaError_t launch_adj_last(const HqChain* chains, int n, int b, cudaStream_t st
   k_adj_last<<<n, HQ_THREADS, 0, st>>>(chains, n, b);
   return cudaGetLastError();
 }
-cudaError_t launch_dyn_commit(const HqChain* chains, int n, int b, cudaStream_t st) {
-  k_dyn_commit<<<n, HQ_THREADS, 0, st>>>(chains, n, b);
+cudaError_t launch_dyn_commit(const HqChain* chains, int n, int b, int Nmax, cudaStream_t st) {
+  const int parts = std::max(1, std::min(8, Nmax * Nmax / 4096));
+  k_dyn_commit<<<dim3(n, parts), HQ_THREADS, 0, st>>>(chains, n, b);
   return cudaGetLastError();
 }
 

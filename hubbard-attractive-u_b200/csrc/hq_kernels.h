@@ -27,9 +27,8 @@ cudaError_t launch_gemm(const HqGemmJob* jobs, int njobs, int Mmax, int Nmax, cu
 cudaError_t launch_measure(const HqChain* chains, int n, int dir, int b, int flags, cudaStream_t st);
 cudaError_t launch_dyn_start(const HqChain* chains, int n, cudaStream_t st);
 cudaError_t launch_dyn_slices(const HqChain* chains, int n, int b, int flags, int Nmax, bool resident, cudaStream_t st);
-cudaError_t launch_dyn_measure(const HqChain* chains, int n, int b, int last_only, cudaStream_t st);
-cudaError_t launch_dyn_store(const HqChain* chains, int n, int b, cudaStream_t st);
-cudaError_t launch_dyn_commit(const HqChain* chains, int n, int b, cudaStream_t st);
+cudaError_t launch_dyn_measure(const HqChain* chains, int n, int b, int pace, cudaStream_t st);
+cudaError_t launch_dyn_commit(const HqChain* chains, int n, int b, int Nmax, cudaStream_t st);
 cudaError_t launch_gather_acc(const HqChain* chains, int n, double* out, cudaStream_t st);
 // the per-chain kernels that live in their own translation units (for function attributes)
 const void* fn_interval();
@@ -61,6 +60,9 @@ cudaError_t launch_sweep(const HqChain* chains, int nchains, const int2* cinfo, 
                          const HqGemmJob* const* lists, int nstab_max, int dir, int flags, int* ctl,
                          unsigned long long* clk, int grid, int Nmax, int kmax, cudaStream_t st);
 const void* fn_sweep();
+// G(0,0) of one chain of up to 64 sites in one launch (the description passed by value, temporaries
+// where it points)
+cudaError_t launch_equaltime(const HqChain& chain, cudaStream_t st);
 cudaError_t launch_adj_interval(const HqChain* chains, int n, int b, int Nmax, bool resident, cudaStream_t st);
 // the finish of the log-det adjoint: log|det| per chain (out), the Daleckii-Krein factor between the
 // products of the eigenbasis of K, the results in the caller's layout

@@ -16,12 +16,11 @@ namespace hq {
 //  direction without updates.
 // ---------------------------------------------------------------------------------
 // The B products of interval b applied to the top of the pushing stack (X = U_top D_top, or 1),
-// into ch.X. `smem` is the dynamic region (N x smem_ld(N) when resident, then the stage and N words); s holds
-// N fields (shared). keep_x (resident only): X stays at the start of `smem` (leading dimension
+// into ch.X. `smem` is the dynamic region (N x smem_ld(N) when resident, then the stage and N words).
+// keep_x (resident only): X stays at the start of `smem` (leading dimension
 // smem_ld(N)) for the factorisation that follows in the same block, instead of going to ch.X.
 // Every thread of the block calls it; the chain is active and b < n_stab.
-__device__ __forceinline__ void bchain_body(const HqChain& ch, int dir, int b, bool resident, double* smem, int8_t* s,
-                                            bool keep_x = false) {
+__device__ __forceinline__ void bchain_body(const HqChain& ch, int dir, int b, bool resident, double* smem, bool keep_x = false) {
   const int N = ch.N;
   int t_lo, t_hi;
   interval_range(ch.nt, ch.pace, ch.n_stab, dir, b, t_lo, t_hi);
@@ -50,20 +49,26 @@ __device__ __forceinline__ void bchain_body(const HqChain& ch, int dir, int b, b
   }
   __syncthreads();
   const int nsl = t_hi - t_lo + 1;
+  // e^{V} of a slice from its fields; the next slice's fields are on their way meanwhile (a slice of a
+  // small lattice takes less time than the load)
+  auto slice = [&](int step) { return ((dir == HQ_DOWN) ? (t_hi - step) : (t_lo + step)) % ch.nt; };
+  auto field = [&](int step) {
+    return step < nsl && (int)threadIdx.x < N ? ch.fields[(size_t)slice(step) * N + threadIdx.x] : (int8_t)0;
+  };
+  int8_t next = field(0);
   for (int step = 0; step < nsl; ++step) {
-    const int t = (dir == HQ_DOWN) ? (t_hi - step) : (t_lo + step);
-    const int l = t % ch.nt;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) s[i] = ch.fields[(size_t)l * N + i];
+    if ((int)threadIdx.x < N) v[threadIdx.x] = next > 0 ? ch.ev_p : ch.ev_m;
+    for (int i = threadIdx.x + blockDim.x; i < N; i += blockDim.x)
+      v[i] = ch.fields[(size_t)slice(step) * N + i] > 0 ? ch.ev_p : ch.ev_m;
+    next = field(step + 1);
     __syncthreads();
     // e^{V} rides on the first pass (down: before expK) or the last pass (up: after it)
-    slice_factors(ch, s, v, nullptr);
-    __syncthreads();
     if (resident) {
-      if (dir == HQ_DOWN) apply_side<LEFT_BT, true, 0>(ch, X, ld, v, stage);
-      else apply_side<LEFT_B, true, 0>(ch, X, ld, v, stage);
+      if (dir == HQ_DOWN) apply_side<LEFT_BT, true>(ch, X, ld, v, stage);
+      else apply_side<LEFT_B, true>(ch, X, ld, v, stage);
     } else {
-      if (dir == HQ_DOWN) apply_side<LEFT_BT, false, 0>(ch, X, ld, v, stage);
-      else apply_side<LEFT_B, false, 0>(ch, X, ld, v, stage);
+      if (dir == HQ_DOWN) apply_side<LEFT_BT, false>(ch, X, ld, v, stage);
+      else apply_side<LEFT_B, false>(ch, X, ld, v, stage);
     }
   }
   if (resident && !keep_x) copy_mat(ch.X, N, X, ld, N);

@@ -191,8 +191,6 @@ __device__ __noinline__ void sep_one(double* M, int ld, const double* coef, doub
 }
 
 // calls f(integral constant L) for the lattice size L in [1, HQ_MAX_L]
-template <int V>
-struct IntC { static constexpr int value = V; };
 template <class F>
 __device__ __forceinline__ void for_lattice(int L, F&& f) {
   switch (L) {

@@ -113,7 +113,7 @@ __device__ int2 take_item(const int2* __restrict__ cinfo, int nchains, int nitem
   return make_int2(-2, 0);
 }
 
-// doubles of the B-chain region (matrix + stage), after which its fields of one slice sit
+// doubles of the B-chain region (matrix, stage, factors of a slice)
 __host__ __device__ inline size_t bchain_doubles(int N) {
   return (size_t)N * smem_ld(N) + 8 * (pad16(N) + 4) + N + 64;
 }
@@ -124,8 +124,11 @@ k_sweep(const HqChain* __restrict__ chains, int nchains, const int2* __restrict_
         unsigned long long* clk) {
   extern __shared__ __align__(16) double smem[];
   __shared__ HqChain ch;
-  __shared__ PivotMoves mv;
-  __shared__ double red[96];
+  // the factorisation's column moves share the words of the reductions (at 144 sites the push leaves
+  // 2.4 KB of the block's shared memory to the static variables)
+  __shared__ __align__(16) double red[96];
+  static_assert(sizeof(PivotMoves) <= sizeof(red), "aliased");
+  PivotMoves& mv = *reinterpret_cast<PivotMoves*>(red);
   __shared__ double pv[2];
   __shared__ int2 s_item;
   __shared__ HqGemmJob jobs[5];
@@ -190,7 +193,7 @@ k_sweep(const HqChain* __restrict__ chains, int nchains, const int2* __restrict_
     mark(1);
     // ---- stack push: B chain, UDV factorisation, cumulative V^T ----
     // X = B ... B U_top D_top stays in shared memory for the factorisation
-    bchain_body(ch, dir, b, true, smem, reinterpret_cast<int8_t*>(smem + bchain_doubles(N)), true);
+    bchain_body(ch, dir, b, true, smem, true);
     __syncthreads();
     mark(2);
     udt_body<2>(ch, side, b, true, smem, mv, true);
@@ -225,7 +228,7 @@ size_t sweep_ctl_ints(int nchains) { return 3 + 2 * (size_t)nchains; }
 // dynamic shared memory of k_sweep for chains of up to Nmax sites and delay depth kmax
 size_t smem_sweep_bytes(int Nmax, int kmax) {
   size_t d = ((interval_smem_doubles(Nmax, kmax, true) + 1) & ~size_t(1)) * sizeof(double) + kIntervalScratchBytes;
-  d = std::max(d, bchain_doubles(Nmax) * sizeof(double) + HQ_MAX_N);
+  d = std::max(d, bchain_doubles(Nmax) * sizeof(double));
   d = std::max(d, smem_udt_bytes(Nmax, true));
   d = std::max(d, smem_invert_bytes(Nmax, true));
   d = std::max(d, cta_gemm_doubles(Nmax, Nmax) * sizeof(double));

@@ -67,8 +67,8 @@ __device__ __forceinline__ bool row_ok(int t, int r, int N) {
 // Reflector of column c (dlarfg convention) by the warp that holds the column in registers; writes
 // the column (R entries, beta, v) and tau[c]. Straight code: a zero column below the diagonal (xs =
 // 0) takes tau = 0 and the factor 1 by selection.
-template <int RPL>
-__device__ __forceinline__ void reflector_reg(double* A, int ld, int N, int c, double (&x)[RPL], double* tau) {
+template <int RPL, bool VB>
+__device__ __forceinline__ void reflector_reg(double* A, int ld, int N, int c, double (&x)[RPL], double* tau, double* vbuf) {
   const int lane = threadIdx.x & 31;
   // two partial sums: the lane's part of the reflector's dependency chain is half as long
   double xs0 = 0.0, xs1 = 0.0, alpha = 0.0;
@@ -93,18 +93,23 @@ __device__ __forceinline__ void reflector_reg(double* A, int ld, int N, int c, d
   for (int t = 0; t < RPL; ++t) {
     const int r = lane + 32 * t;
     x[t] = (r == c) ? beta : (r > c ? x[t] * rs : x[t]);
-    if (row_ok<RPL>(t, r, N)) Ac[r] = x[t];
+    if (row_ok<RPL>(t, r, N)) {
+      Ac[r] = x[t];
+      if (VB) vbuf[r] = x[t];
+    }
   }
   tau[c] = ti;  // every lane the same value
 }
 
+// VB: A is in global memory, and the reflectors pass between the warps through two shared buffers of
+// 256 words (vbuf, vbuf + 256) instead.
 // Householder QR of the panel columns [p0, p1) for N <= 32 RPL: the panel's kQB columns are held
 // in registers, CPW per warp by kQB / CPW warps (warp w holds columns p0 + w + i kQB / CPW);
 // the owner of column c+1 forms reflector c+1 right after applying reflector c, so one block
 // barrier separates consecutive reflectors. Bound by that chain (two warp sums, a square root and
 // two reciprocals per column). RPL = ceil(N / 32): 16 x 16 matrices took the time of five row slots.
-template <int RPL, int CPW>
-__device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* tau) {
+template <int RPL, int CPW, bool VB = false>
+__device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* tau, double* vbuf = nullptr) {
   constexpr int NWP = kQB / CPW;  // warps that hold panel columns
   const int lane = threadIdx.x & 31, warp = warp_index();
   int col[CPW];
@@ -120,7 +125,7 @@ __device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* t
       x[i][t] = (own[i] && row_ok<RPL>(t, r, N)) ? A[r + (size_t)col[i] * ld] : 0.0;
     }
   }
-  if (warp == 0) reflector_reg<RPL>(A, ld, N, p0, x[0], tau);
+  if (warp == 0) reflector_reg<RPL, VB>(A, ld, N, p0, x[0], tau, vbuf + 256 * (p0 & 1));
   __syncthreads();
   for (int c = p0; c + 1 < p1; ++c) {
 #pragma unroll
@@ -132,7 +137,7 @@ __device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* t
 #pragma unroll
         for (int t = 0; t < RPL; ++t) {
           const int r = lane + 32 * t;
-          const double vr = row_ok<RPL>(t, r, N) ? A[r + (size_t)c * ld] : 0.0;
+          const double vr = row_ok<RPL>(t, r, N) ? (VB ? vbuf[256 * (c & 1) + r] : A[r + (size_t)c * ld]) : 0.0;
           v[t] = r > c ? vr : (r == c ? 1.0 : 0.0);
           if (t & 1) w1 = fma(v[t], x[i][t], w1);
           else w0 = fma(v[t], x[i][t], w0);
@@ -140,7 +145,7 @@ __device__ void qr_panel_reg(double* A, int ld, int N, int p0, int p1, double* t
         const double w = warp_sum(w0 + w1) * ti;
 #pragma unroll
         for (int t = 0; t < RPL; ++t) x[i][t] = fma(-w, v[t], x[i][t]);
-        if (col[i] == c + 1) reflector_reg<RPL>(A, ld, N, c + 1, x[i], tau);
+        if (col[i] == c + 1) reflector_reg<RPL, VB>(A, ld, N, c + 1, x[i], tau, vbuf + 256 * ((c + 1) & 1));
       }
     }
     __syncthreads();
@@ -494,7 +499,9 @@ __device__ __forceinline__ void udt_body(const HqChain& ch, int side, int b, boo
       constexpr int RPL = decltype(rc)::value;
       panel_pivot<RPL>(A, ld, N, p0, p1, nrm, order, rk, Vb, ldp, mv);
       phase(1);
-      if constexpr (RPL > 0) qr_panel_reg<RPL, CPW>(A, ld, N, p0, p1, tau);
+      // (T and S, 256 words each, are free until the panel's T factor)
+      if constexpr (RPL > 5) qr_panel_reg<RPL, CPW, true>(A, ld, N, p0, p1, tau, T);
+      else if constexpr (RPL > 0) qr_panel_reg<RPL, CPW>(A, ld, N, p0, p1, tau);
       else qr_panel(A, ld, N, p0, p1, tau);
     };
     if (N <= 32) panel(IntC<1>{});
@@ -502,7 +509,18 @@ __device__ __forceinline__ void udt_body(const HqChain& ch, int side, int b, boo
     else if (N <= 96) panel(IntC<3>{});
     else if (N <= 128) panel(IntC<4>{});
     else if (N <= 160) panel(IntC<5>{});
-    else panel(IntC<0>{});
+    else {
+      // sizes beyond one SM's shared memory (16 warps): up to 256 rows the panel is in registers all
+      // the same; an unblocked panel in global memory waits on L2 several times per column
+      if constexpr (CPW == 1) {
+        if (N <= 192) panel(IntC<6>{});
+        else if (N <= 224) panel(IntC<7>{});
+        else if (N <= 256) panel(IntC<8>{});
+        else panel(IntC<0>{});
+      } else {
+        panel(IntC<0>{});
+      }
+    }
     phase(2);
     if (p1 < N) {
       double* Tp = Tc + (size_t)(p0 / kQB) * kQB * kQB;

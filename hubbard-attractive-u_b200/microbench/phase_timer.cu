@@ -180,7 +180,7 @@ static void time_udt(const std::vector<double>& h, double* X, double* U, double*
   const size_t NN = (size_t)kN * kN;
   cudaMemset(clk, 0, kSlots * 8);
   // the dynamic shared memory of k_udt (smem_udt_bytes, resident)
-  const size_t smem = ((size_t)kN * smem_ld(kN) + 2 * kQB * panel_ld(kN) + 2 * kQB * kQB + 3 * kN + 64 +
+  const size_t smem = ((size_t)kN * smem_ld(kN) + 2 * kQB * panel_ld(kN) + 2 * kQB * kQB + 3 * kN +
                        ((kN - 1) / kQB) * kQB * kQB) * 8;
   cudaFuncSetAttribute(k_udt_phases<CPW, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_udt_phases<CPW, NT><<<nb, NT, smem>>>(X, U, D, T, clk);
