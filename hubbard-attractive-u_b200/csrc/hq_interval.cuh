@@ -37,6 +37,10 @@ __device__ __forceinline__ MetroShared metro_shared(double* smem, const Interval
 template <int L>
 __device__ __noinline__ int metropolis_slice(const HqChain& ch, uint32_t rng, int flags, long long log_base) {
   extern __shared__ __align__(16) double smem[];
+  // Warp 0 walks the next block beside the flush where the flush is long: 16 x 24 strips for seven warps
+  // from 100 sites on. With G in global memory it is so long that a warp less costs more than the walk
+  // beside it saves (14 x 14: 17.9 against 16.7 ms a sweep of 16 chains).
+  constexpr bool kAhead = L >= 10;
   const int N = L > 0 ? L * L : ch.N;
   const IntervalLayout lay = interval_layout(N, L > 0 ? 16 : ch.kmax, L > 0);
   const MetroShared sh = metro_shared(smem, lay, N);
@@ -44,7 +48,7 @@ __device__ __noinline__ int metropolis_slice(const HqChain& ch, uint32_t rng, in
   const int ld = L > 0 ? interval_ld(N) : N;
   const int ldp = panel_ld(pad16(N));
   const int NB = ch.kmax;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = kAhead ? warp_index() : tid >> 5;
   const bool log = (flags & HQ_F_LOG_RATIOS) && ch.ratios;
   // uniforms of this slice: site i consumes engine draws 2i+1, 2i+2 after the current state
   for (int i = tid; i < N; i += blockDim.x) {
@@ -57,22 +61,52 @@ __device__ __noinline__ int metropolis_slice(const HqChain& ch, uint32_t rng, in
   }
   __syncthreads();
   int acc_count = 0;
-  for (int b0 = 0, bi = 0; b0 < N; b0 += NB, ++bi) {
-    if (warp == 0) walk(G, ld, sh, b0, min(NB, N - b0), log, bi & 1);
+  if constexpr (kAhead) {
+    // bn: the block to walk; the one before it is to flush. The walk stands in the code once (with a copy
+    // per flip count the instruction cache ate half of the gain).
+    for (int bn = 0, bi = 0;; bn += NB, ++bi) {
+      const bool more = bn < N, ahead = more && warp == 0;
+      int a = 0;
+      if (bn > 0) {
+        __syncthreads();  // the previous block's walk and the flush before it are done
+        // the count alternates between two words: with no flush (a == 0) no barrier follows,
+        // and warp 0 writes the next block's count while other warps may still read this one
+        a = sh.ired[(bi - 1) & 1];
+        acc_count += a;
+      }
+      NextTile next;
+      if (ahead) next.load(G + bn + (size_t)bn * ld, ld, min(NB, N - bn));
+      if (a > 0)
+        for_ksteps(a, [&](auto kc) {
+          constexpr int KA = decltype(kc)::value;
+          build_panels<KA>(G, ld, N, sh, ldp, a, bn - NB);
+          __syncthreads();
+          if (ahead) next.update<KA>(sh.X + bn, ldp, sh.Y + bn, ldp);
+          else rank_strips<pad16(L * L) / 16, tile_cols(L * L), KA>(G, ld, sh, ldp, ldp, more ? warp - 1 : warp, more ? 7 : 8);
+        });
+      if (!more) break;
+      if (ahead) {
+        next.store(sh.xt);
+        walk(sh.xt, kLdR, sh, bn, min(NB, N - bn), log, bi & 1, [&] { next.store(sh.xt); });
+      }
+    }
     __syncthreads();
-    // the count alternates between two words: with no flush (a == 0) no barrier follows,
-    // and warp 0 writes the next block's count while other warps may still read this one
-    const int a = sh.ired[bi & 1];
-    acc_count += a;
-    if (a == 0) continue;
-    for_ksteps(a, [&](auto kc) {
-      constexpr int KA = decltype(kc)::value;
-      build_panels<KA>(G, ld, N, sh, ldp, a, b0);
+  } else {
+    for (int b0 = 0, bi = 0; b0 < N; b0 += NB, ++bi) {
+      if (warp == 0) walk(G + b0 + (size_t)b0 * ld, ld, sh, b0, min(NB, N - b0), log, bi & 1);
       __syncthreads();
-      if constexpr (L > 0) rank_strips<pad16(L * L) / 16, tile_cols(L * L), KA>(G, ld, sh, ldp, ldp);
-    });
-    if constexpr (L == 0) rank_update48(G, ld, N, N, sh, ldp, ldp, a);
-    __syncthreads();
+      const int a = sh.ired[bi & 1];  // alternating words, as above
+      acc_count += a;
+      if (a == 0) continue;
+      for_ksteps(a, [&](auto kc) {
+        constexpr int KA = decltype(kc)::value;
+        build_panels<KA>(G, ld, N, sh, ldp, a, b0);
+        __syncthreads();
+        if constexpr (L > 0) rank_strips<pad16(L * L) / 16, tile_cols(L * L), KA>(G, ld, sh, ldp, ldp, tid >> 5, HQ_INT_THREADS / 32);
+      });
+      if constexpr (L == 0) rank_update48(G, ld, N, N, sh, ldp, ldp, a);
+      __syncthreads();
+    }
   }
   // apply the flips of this slice and optionally log the visit-time ratios
   for (int i = tid; i < N; i += blockDim.x) {

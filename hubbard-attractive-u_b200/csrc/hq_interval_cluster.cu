@@ -131,7 +131,7 @@ __device__ __forceinline__ void cl_wrap(const HqChain& ch, double* Gc, double* c
 __device__ __forceinline__ void cl_metropolis(const HqChain& ch, double* Gc, int rank, int c0, MetroShared& sh, double* u_l,
                                               double* thr_l, double* dl_l, int8_t* flip_l, const uint32_t* pw,
                                               uint32_t& rng, double& n_acc, bool log, cg::cluster_group& cluster) {
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_index();
   double* Gs = Gc - (size_t)c0 * kLd;  // absolute column index -> local storage
   for (int q = tid; q < kNC; q += blockDim.x) {
     const uint32_t x1 = minstd_mulmod(pw[q], rng);
@@ -145,40 +145,50 @@ __device__ __forceinline__ void cl_metropolis(const HqChain& ch, double* Gc, int
   rng = minstd_mulmod(minstd_pow(2ull * kN), rng);
   __syncthreads();
   double acc_count = 0.0;
-  for (int b0 = 0, bi = 0; b0 < kN; b0 += 16, ++bi) {
-    const int owner = b0 / kNC;
-    const int slot = bi & 1;
-    if (rank == owner && warp == 0) walk(Gs, kLd, sh, b0, 16, log, slot);
-    cluster.sync();  // the walk's records are visible to the cluster
-    const int* o_ired = cluster.map_shared_rank(sh.ired, owner);
-    const int a = o_ired[slot];
-    if (rank == owner && tid == 0) acc_count += a;
-    if (a == 0) continue;
-    if (rank != owner) {
-      const double* orec = cluster.map_shared_rank(sh.xt, owner);
-      const int* oqj = cluster.map_shared_rank(sh.qj, owner);
-      for (int k = tid; k < kRecordDoubles; k += blockDim.x) sh.xt[k] = orec[k];
-      if (tid < 16) sh.qj[tid] = oqj[tid];
-      __syncthreads();
+  // bn: the block to walk, by warp 0 of its owner; the one before it is to flush
+  for (int bn = 0, bi = 0;; bn += 16, ++bi) {
+    const bool next_here = bn < kN && rank == bn / kNC, ahead = next_here && warp == 0;
+    const int b0 = bn - 16, owner = bn > 0 ? b0 / kNC : 0;
+    int a = 0;
+    if (bn > 0) {
+      cluster.sync();  // the previous block's walk is visible to the cluster, the flushes before it are done
+      a = cluster.map_shared_rank(sh.ired, owner)[(bi - 1) & 1];
+      if (rank == owner && tid == 0) acc_count += a;
     }
-    for_ksteps(a, [&](auto kc) {
-      constexpr int KA = decltype(kc)::value;
-      if (tid >= 128) panel_cols<KA>(Gc + b0, kLd, kNC, c0, sh, a, b0, kLdy);
-      else if (rank == owner) panel_rows<KA>(Gs + (size_t)b0 * kLd, kLd, kN, sh, a, kLdx);
-      cluster.sync();  // X is complete in the owner's shared memory
+    NextTile next;
+    if (ahead) next.load(Gs + bn + (size_t)bn * kLd, kLd, 16);
+    if (a > 0) {
       if (rank != owner) {
-        const double* oX = cluster.map_shared_rank(sh.X, owner);
-        static_assert(HQ_INT_THREADS == kN, "one row of X per thread");
-        double v[4 * KA];
-#pragma unroll
-        for (int m = 0; m < 4 * KA; ++m) v[m] = oX[tid + m * kLdx];
-#pragma unroll
-        for (int m = 0; m < 4 * KA; ++m) sh.X[tid + m * kLdx] = v[m];
+        const double* orec = cluster.map_shared_rank(sh.xt, owner);
+        const int* oqj = cluster.map_shared_rank(sh.qj, owner);
+        for (int k = tid; k < kRecordDoubles; k += blockDim.x) sh.xt[k] = orec[k];
+        if (tid < 16) sh.qj[tid] = oqj[tid];
+        __syncthreads();
       }
-      __syncthreads();
-      rank_strips<kN / 16, kNC / 8, KA>(Gc, kLd, sh, kLdx, kLdy);
-    });
-    __syncthreads();
+      for_ksteps(a, [&](auto kc) {
+        constexpr int KA = decltype(kc)::value;
+        if (tid >= 128) panel_cols<KA>(Gc + b0, kLd, kNC, c0, sh, a, b0, kLdy);
+        else if (rank == owner) panel_rows<KA>(Gs + (size_t)b0 * kLd, kLd, kN, sh, a, kLdx);
+        cluster.sync();  // X is complete in the owner's shared memory
+        if (rank != owner) {
+          const double* oX = cluster.map_shared_rank(sh.X, owner);
+          static_assert(HQ_INT_THREADS == kN, "one row of X per thread");
+          double v[4 * KA];
+#pragma unroll
+          for (int m = 0; m < 4 * KA; ++m) v[m] = oX[tid + m * kLdx];
+#pragma unroll
+          for (int m = 0; m < 4 * KA; ++m) sh.X[tid + m * kLdx] = v[m];
+        }
+        __syncthreads();
+        if (ahead) next.update<KA>(sh.X + bn, kLdx, sh.Y + bn - c0, kLdy);
+        else rank_strips<kN / 16, kNC / 8, KA>(Gc, kLd, sh, kLdx, kLdy, next_here ? warp - 1 : warp, next_here ? 7 : 8);
+      });
+    }
+    if (bn >= kN) break;
+    if (ahead) {
+      next.store(sh.xt);
+      walk(sh.xt, kLdR, sh, bn, 16, log, bi & 1, [&] { next.store(sh.xt); });
+    }
   }
   n_acc += acc_count;
   cluster.sync();  // every walk of the slice is done: the flip flags are final

@@ -26,11 +26,16 @@ namespace hq {
 //        Y[m, :] = G[j_m, :] - e_{j_m}^T + sum_{m'<m} X[j_m, m'] Y[m', :]
 //      one row of X and one column of Y per thread, with the coefficients X[B, :] and
 //      Y[:, B] from the walk's records;
-//   3. G += X Y by DMMA (rank a <= 16) over all warps.
-//  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 40, 18, 46;
-//  56, 28 and 85 with predicated record stores and a reciprocal with range checks in the walk, a
-//  branch per flip in the panels, and a flush that checked every element against the edge. The
-//  walk and the panels are bound by the latency of one dependency chain, the flush by the DMMA pipe.
+//   3. G += X Y by DMMA (rank a <= 16).
+//  On lattices of 100 sites and more with G in shared memory, warps 1 .. 7 flush while warp 0 takes the
+//  next block's g = G[B', B'] + X[B', :] Y[:, B'] (the same DMMA steps, so the same bits as the flush
+//  leaves) and walks it.
+//  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 40, 18, 46 one
+//  after the other; 56, 28 and 85 with predicated record stores and a reciprocal with range checks in
+//  the walk, a branch per flip in the panels, and a flush that checked every element against the edge.
+//  The walk and the panels are bound by the latency of one dependency chain, the flush by the DMMA
+//  pipe. With the walks beside the flushes a round trip of 200 slices at 12 x 12 takes 256 chains
+//  56.3 ms instead of 60.5, one chain 23.0 instead of 25.5.
 // ---------------------------------------------------------------------------------
 constexpr int kLdR = 18;  // leading dimension of the walk's records: 16-byte rows whose stores spread over the banks
 
@@ -59,8 +64,8 @@ __device__ __forceinline__ double reference_ratio(double gii, double dl) {
   return __ddiv_rn(__dmul_rn(a, a), __dadd_rn(1.0, dl));
 }
 
-// The walk of the nb <= 16 sites [b0, b0 + nb) by one warp. Lane 8 rg + cg holds the entries
-// (4 rg + a, 2 cg + b), a < 4, b < 2, of g: a step needs column s at the lane's four rows, row s at its
+// The walk of the nb <= 16 sites [b0, b0 + nb) by one warp, from their tile g of G. Lane 8 rg + cg
+// holds the entries (4 rg + a, 2 cg + b), a < 4, b < 2, of g: a step needs column s at the lane's four rows, row s at its
 // two columns and the diagonal entry, 7 shuffles. Entries of rows and columns already visited are
 // not read again; they are left to run along.
 //
@@ -68,7 +73,7 @@ __device__ __forceinline__ double reference_ratio(double gii, double dl) {
 // u (1 + Delta) < a^2 (1 + Delta > 0), which needs no division on its dependency chain and equals
 // the reference's test except when the two sides lie within a few rounding errors of each other.
 // It only records whether that happened (warp-uniform; probability ~1e-12 per proposal): the
-// return value. The caller then walks the block again, from its unchanged G, with EXACT: every
+// return value. The caller then walks the block again, from its unchanged g, with EXACT: every
 // decision in the reference's own form, u < min(1, |r|) with r as the reference evaluates it.
 // The one warp issues in order, so the walk is straight code: every lane stores its records (lanes
 // without any to a spare word), of accepted sites and others alike (the next site's overwrite them),
@@ -76,7 +81,7 @@ __device__ __forceinline__ double reference_ratio(double gii, double dl) {
 // per block); the sites' constants are in registers before the first store (3.2k -> 2.9k); and
 // NBC = 16 fixes nb at compile time (NBC = 0 takes nb). LOGT false compiles the ratio log out.
 template <bool EXACT, bool LOGT, int NBC>
-__device__ __forceinline__ bool walk_block16(const double* G, int ld, const MetroShared& sh, int b0, int nbr, int slot) {
+__device__ __forceinline__ bool walk_block16(const double* g, int ld, const MetroShared& sh, int b0, int nbr, int slot) {
   constexpr int NB = 16;
   const int nb = NBC > 0 ? NBC : nbr;
   const int lane = threadIdx.x & 31;
@@ -87,8 +92,9 @@ __device__ __forceinline__ bool walk_block16(const double* G, int ld, const Metr
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       const int row = 4 * rg + a, col = 2 * cg + b;
-      r[a][b] = (row < nb && col < nb) ? G[b0 + row + (size_t)(b0 + col) * ld] : 0.0;
+      r[a][b] = (row < nb && col < nb) ? g[row + (size_t)col * ld] : 0.0;
     }
+  __syncwarp();
   double dls[NB], thrs[NB];
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
@@ -155,19 +161,62 @@ __device__ __forceinline__ bool walk_block16(const double* G, int ld, const Metr
 // the walks of the ratio log, of near ties and of short blocks, out of line: their code and
 // registers do not weigh on the fast walk's
 template <bool EXACT, bool LOGT>
-__device__ __noinline__ bool walk_rare(const double* G, int ld, const MetroShared sh, int b0, int nb, int slot) {
-  return walk_block16<EXACT, LOGT, 0>(G, ld, sh, b0, nb, slot);
+__device__ __noinline__ bool walk_rare(const double* g, int ld, const MetroShared sh, int b0, int nb, int slot) {
+  return walk_block16<EXACT, LOGT, 0>(g, ld, sh, b0, nb, slot);
 }
-// the walk with the reference's form of every decision where the fast one came near a tie
-__device__ __forceinline__ void walk(const double* G, int ld, const MetroShared& sh, int b0, int nb, bool log, int slot) {
+// the walk with the reference's form of every decision where the fast one came near a tie; again()
+// restores g before a second walk, if the first one's records overwrote it
+template <class F>
+__device__ __forceinline__ void walk(const double* g, int ld, const MetroShared& sh, int b0, int nb, bool log, int slot, F&& again) {
   if (log) {
-    if (walk_rare<false, true>(G, ld, sh, b0, nb, slot)) walk_rare<true, true>(G, ld, sh, b0, nb, slot);
+    if (walk_rare<false, true>(g, ld, sh, b0, nb, slot)) again(), walk_rare<true, true>(g, ld, sh, b0, nb, slot);
   } else if (nb == 16) {
-    if (walk_block16<false, false, 16>(G, ld, sh, b0, nb, slot)) walk_rare<true, false>(G, ld, sh, b0, nb, slot);
+    if (walk_block16<false, false, 16>(g, ld, sh, b0, nb, slot)) again(), walk_rare<true, false>(g, ld, sh, b0, nb, slot);
   } else {
-    if (walk_rare<false, false>(G, ld, sh, b0, nb, slot)) walk_rare<true, false>(G, ld, sh, b0, nb, slot);
+    if (walk_rare<false, false>(g, ld, sh, b0, nb, slot)) again(), walk_rare<true, false>(g, ld, sh, b0, nb, slot);
   }
 }
+// the walk of a tile that lies in G
+__device__ __forceinline__ void walk(const double* g, int ld, const MetroShared& sh, int b0, int nb, bool log, int slot) {
+  walk(g, ld, sh, b0, nb, log, slot, [] {});
+}
+
+// The next block's tile for the walk beside the flush, in DMMA accumulators of warp 0: the nb x nb
+// entries at g, loaded before the flush touches G; then the flush's own k-steps (the block's rows of
+// X, its columns of Y); then into shared memory, where it takes the place of the records xt: the walk has
+// read it before its first record is written (a tile of its own would take 2.3 KB from the L1 cache).
+struct NextTile {
+  double v[2][4];
+  __device__ __forceinline__ void load(const double* g, int ld, int nb) {
+    const int gr = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = gr + ((e & 2) ? 8 : 0), col = 8 * t + 2 * q + (e & 1);
+        v[t][e] = (row < nb && col < nb) ? g[row + (size_t)col * ld] : 0.0;
+      }
+  }
+  template <int KA>
+  __device__ __forceinline__ void update(const double* Xr, int ldx, const double* Yc, int ldy) {
+    const int gr = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+#pragma unroll
+    for (int s = 0; s < KA; ++s) {
+      const double a0 = Xr[gr + (4 * s + q) * ldx], a1 = Xr[gr + 8 + (4 * s + q) * ldx];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) dmma_16x8x4(v[t], a0, a1, Yc[(4 * s + q) * ldy + 8 * t + gr]);
+    }
+  }
+  __device__ __forceinline__ void store(double* tile) const {
+    const int gr = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) tile[gr + ((e & 2) ? 8 : 0) + (8 * t + 2 * q + (e & 1)) * kLdR] = v[t][e];
+    __syncwarp();
+  }
+};
 
 // W lines of a panel for a flips, 4 (KA - 1) < a <= 4 KA, in the thread's registers,
 //   v[m] = w_m (g[m] + sum_{m'<m} c[j_m][m'] v[m']):
@@ -332,16 +381,15 @@ __device__ __forceinline__ void rank_update48(double* G, int ld, int M, int Nc, 
 // Bound by the DMMA pipe (12 x 12, rank 12: 162 tiles x 3 steps x 8 cycles = 3.9k of 5.2k
 // measured); strips of 16 x 24 keep eight warps evenly loaded (54 strips), 48 x 32 tiles took 7.1k.
 template <int MT, int T, int KS>
-__device__ __forceinline__ void rank_strips(double* G, int ld, const MetroShared& sh, int ldx, int ldy) {
+__device__ __forceinline__ void rank_strips(double* G, int ld, const MetroShared& sh, int ldx, int ldy, int warp, int nw) {
   constexpr int NT = T % 3 == 0 ? 3 : 2;
-  constexpr int NG = T / NT;
   static_assert(T % NT == 0, "tile_cols pads the columns to whole strips");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int g = lane >> 2, q = lane & 3;
   const double* Xq = sh.X + q * ldx + g;
   const double* Yq = sh.Y + q * ldy + g;
 #pragma unroll 1
-  for (int st = warp; st < MT * NG; st += nw) {
+  for (int st = warp; st < MT * (T / NT); st += nw) {
     const int r0 = (st % MT) * 16, t0 = (st / MT) * NT;
     double* Gp = G + r0 + g + (size_t)(8 * t0 + 2 * q) * ld;
     const double* Yp = Yq + 8 * t0;

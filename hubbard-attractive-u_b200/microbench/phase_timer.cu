@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(HQ_INT_THREADS, 1) k_flush(unsigned long long*
   __syncthreads();
   const long long t0 = clock64();
   for (int r = 0; r < reps; ++r) {
-    for_ksteps(k, [&](auto kc) { rank_strips<pad16(kN) / 16, tile_cols(kN), decltype(kc)::value>(G, ld, sh, ldp, ldp); });
+    for_ksteps(k, [&](auto kc) { rank_strips<pad16(kN) / 16, tile_cols(kN), decltype(kc)::value>(G, ld, sh, ldp, ldp, threadIdx.x >> 5, blockDim.x >> 5); });
     __syncthreads();
   }
   if (threadIdx.x == 0) atomicAdd(clk, (unsigned long long)(clock64() - t0));
