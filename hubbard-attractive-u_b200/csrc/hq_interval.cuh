@@ -37,10 +37,11 @@ __device__ __forceinline__ MetroShared metro_shared(double* smem, const Interval
 template <int L>
 __device__ __noinline__ int metropolis_slice(const HqChain& ch, uint32_t rng, int flags, long long log_base) {
   extern __shared__ __align__(16) double smem[];
-  // Warp 0 walks the next block beside the flush where the flush is long: 16 x 24 strips for seven warps
-  // from 100 sites on. With G in global memory it is so long that a warp less costs more than the walk
-  // beside it saves (14 x 14: 17.9 against 16.7 ms a sweep of 16 chains).
-  constexpr bool kAhead = L >= 10;
+  // Warp 0 walks the next block beside the flush where the flush is long enough to lose a warp: round
+  // trips with / without, ms: 48 chains of 9 x 9 6.48 / 6.67, one of 8 x 8 10.07 / 10.06, 32 of 7 x 7
+  // 5.26 / 5.06. With G in global memory the flush is so long that the warp it lacks costs more than
+  // the walk beside it saves (16 chains of 14 x 14, interval kernel: 17.9 / 16.7 ms a sweep).
+  constexpr bool kAhead = L >= 9;
   const int N = L > 0 ? L * L : ch.N;
   const IntervalLayout lay = interval_layout(N, L > 0 ? 16 : ch.kmax, L > 0);
   const MetroShared sh = metro_shared(smem, lay, N);

@@ -27,7 +27,7 @@ namespace hq {
 //      one row of X and one column of Y per thread, with the coefficients X[B, :] and
 //      Y[:, B] from the walk's records;
 //   3. G += X Y by DMMA (rank a <= 16).
-//  On lattices of 100 sites and more with G in shared memory, warps 1 .. 7 flush while warp 0 takes the
+//  On lattices of 81 sites and more with G in shared memory, warps 1 .. 7 flush while warp 0 takes the
 //  next block's g = G[B', B'] + X[B', :] Y[:, B'] (the same DMMA steps, so the same bits as the flush
 //  leaves) and walks it.
 //  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 40, 18, 46 one
