@@ -62,22 +62,6 @@ __device__ __forceinline__ void dmma_16x8x4(double (&c)[4], double a0, double a1
       : "d"(a0), "d"(a1), "d"(b0));
 }
 
-// ------------------------------------------------------------------------------------
-//  1 / x correctly rounded, for x and 1 / x normal numbers: the hardware's approximation (it reads and
-//  gives 20 mantissa bits), one step y (1 + e + e^2), e = 1 - x y, of the cubic iteration (2^-60 and a
-//  rounding) and one Newton step, whose FMA residual leaves 2^-104 before the last rounding. (Two
-//  Newton steps leave 2^-80: one in 10^8 results is off by an ulp, which large batches meet.)
-//  Without the range checks and the branch of the intrinsic, whose value it has, the code around it
-//  is straight (the walk and the pivots are chains of one warp that issues in order).
-// ------------------------------------------------------------------------------------
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  y = fma(y, fma(e, e, e), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
 // the warp's index as a value the compiler knows to be the same in all its lanes, so that branches
 // on it need no reconvergence
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }

@@ -83,7 +83,7 @@ __device__ __forceinline__ void gj_pivot_reg(double (&x)[RPL], int k, int N, dou
   const int bi = (int)__reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? (unsigned)cr[0] : 0xffffffffu);
   const double vb = __shfl_sync(0xffffffffu, cx[0], bi & 31);  // row bi is the candidate of its lane
   const bool ok = (mh | ml) != 0u && isfinite(vb);
-  const double pinv = ok ? reciprocal(vb) : 0.0;
+  const double pinv = ok ? __drcp_rn(vb) : 0.0;  // 1 / vb, correctly rounded
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
     const int r = lane + 32 * t;

@@ -31,8 +31,8 @@ namespace hq {
 //  next block's g = G[B', B'] + X[B', :] Y[:, B'] (the same DMMA steps, so the same bits as the flush
 //  leaves) and walks it.
 //  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 40, 18, 46 one
-//  after the other; 56, 28 and 85 with predicated record stores and a reciprocal with range checks in
-//  the walk, a branch per flip in the panels, and a flush that checked every element against the edge.
+//  after the other; 56, 28 and 85 with predicated record stores in the walk, a branch per flip in the
+//  panels, and a flush that checked every element against the edge.
 //  The walk and the panels are bound by the latency of one dependency chain, the flush by the DMMA
 //  pipe. With the walks beside the flushes a round trip of 200 slices at 12 x 12 takes 256 chains
 //  56.3 ms instead of 60.5, one chain 23.0 instead of 25.5.
@@ -121,7 +121,7 @@ __device__ __forceinline__ bool walk_block16(const double* g, int ld, const Metr
 #pragma unroll
       for (int b = 0; b < 2; ++b) row[b] = __shfl_sync(0xffffffffu, r[s & 3][b], 8 * (s >> 2) + cg);
       const double av = fma(-dg, dl, 1.0 + dl);  // 1 + (1 - g_ss) Delta
-      const double rc = reciprocal(av);
+      const double rc = __drcp_rn(av);
       const double gam = dl * rc;                // gamma = Delta / av
       if (LOGT && lane == s) myr = reference_ratio(dg, dl);
       bool acc;
