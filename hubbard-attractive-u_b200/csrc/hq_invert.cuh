@@ -80,8 +80,9 @@ __device__ __forceinline__ void gj_pivot_reg(double (&x)[RPL], int k, int N, dou
   const unsigned hi = (unsigned)(bb >> 32), lo = (unsigned)bb;
   const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
   const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  const int bi = (int)__reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? (unsigned)cr[0] : 0xffffffffu);
-  const double vb = __shfl_sync(0xffffffffu, cx[0], bi & 31);  // row bi is the candidate of its lane
+  const int br = (int)__reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? (unsigned)cr[0] : 0xffffffffu);
+  const int bi = br < N ? br : k;  // no candidate (a column of NaNs): row k stays, so that perm holds rows of the matrix
+  const double vb = __shfl_sync(0xffffffffu, cx[0], bi & 31);  // row br is the candidate of its lane
   const bool ok = (mh | ml) != 0u && isfinite(vb);
   const double pinv = ok ? __drcp_rn(vb) : 0.0;  // 1 / vb, correctly rounded
 #pragma unroll
