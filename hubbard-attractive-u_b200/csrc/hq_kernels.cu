@@ -12,6 +12,7 @@
 //                include/observable_methods.hpp:84-195).
 //  k_adj_*     : adjoint of log|det(1 + B...B)| (no counterpart in the reference).
 #include <algorithm>
+#include <mutex>
 
 #include "hq_phases.cuh"
 
@@ -461,13 +462,15 @@ size_t smem_matrix_bytes(int Nmax, bool resident, int extra_doubles) {
 // context of small chains never lowers the limit an existing context of larger chains
 // launches with.
 constexpr int kMaxTrackedDevices = 64;
-constexpr int kTrackedKernels = 9;
+constexpr int kTrackedKernels = 10;
 static size_t g_smem_set[kMaxTrackedDevices][kTrackedKernels];
+static std::mutex g_smem_mutex;  // contexts may be created by several threads at once
 
 static cudaError_t raise_smem(int slot, const void* fn, size_t bytes) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(g_smem_mutex);
   if (dev >= 0 && dev < kMaxTrackedDevices && g_smem_set[dev][slot] >= bytes) return cudaSuccess;
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess && dev >= 0 && dev < kMaxTrackedDevices) g_smem_set[dev][slot] = bytes;
@@ -513,6 +516,8 @@ cudaError_t prepare_interval_cl() {
   if (e != cudaSuccess) return e;
   return raise_smem(7, fn_bchain_cols(), smem_bchain_cols_bytes());
 }
+
+cudaError_t prepare_sweep(int Nmax, int kmax) { return raise_smem(9, fn_sweep(), smem_sweep_bytes(Nmax, kmax)); }
 
 cudaError_t launch_bchain(const HqChain* chains, int n, int dir, int b, int Nmax, bool resident, cudaStream_t st) {
   const size_t bytes = smem_bchain_bytes(Nmax, resident);

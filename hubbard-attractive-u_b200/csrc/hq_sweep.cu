@@ -243,11 +243,6 @@ bool sweep_fits(int Nmax, int kmax, size_t optin) {
   return Nmax <= 160 && a.sharedSizeBytes + smem_sweep_bytes(Nmax, kmax) <= optin;
 }
 
-cudaError_t prepare_sweep(int Nmax, int kmax) {
-  return cudaFuncSetAttribute((const void*)k_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem_sweep_bytes(Nmax, kmax));
-}
-
 cudaError_t launch_sweep(const HqChain* chains, int nchains, const int2* cinfo, int nitems,
                          const HqGemmJob* const* lists, int nstab_max, int dir, int flags, int* ctl,
                          unsigned long long* clk, int grid, int Nmax, int kmax, cudaStream_t st) {

@@ -1,0 +1,40 @@
+"""Several contexts in one process, idle SMs of a small context, and contexts of very many chains."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+UP, DOWN, DYN = 0, 1, 2
+
+
+def _run(hq, e, trips=2):
+    for _ in range(trips):
+        e.sweep(UP, hq.SWEEP_MEASURE)
+        e.sweep(DOWN, hq.SWEEP_MEASURE)
+    e.sync()
+    return [e.g(0), e.fields(0), e.estimators(0)]
+
+
+@pytest.mark.parametrize("mode", [0, 1], ids=["launches", "persistent"])
+def test_a_context_of_smaller_chains_beside_a_larger_one(hq, mode):
+    """The kernels' shared-memory limits are shared by the contexts of a process: a later context of
+    smaller chains leaves them where an earlier one needs them."""
+    def make(L):
+        e = hq.Engine([dict(nl=L, u=4.0, mu=0.1, beta=0.8, nt=8, stabilization_pace=5, seed=L)])
+        e.set_sweep_mode(mode)
+        e.fields_random()
+        e.init()
+        return e
+    a = make(12)
+    want = _run(hq, a)
+    a.close()
+    a = make(12)
+    b = make(4)
+    got_small = _run(hq, b)
+    for x, y in zip(_run(hq, a), want):
+        assert np.array_equal(x, y)
+    c = make(4)
+    for x, y in zip(_run(hq, c), got_small):
+        assert np.array_equal(x, y)
+    for e in (a, b, c):
+        e.close()
