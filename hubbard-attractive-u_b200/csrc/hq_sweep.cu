@@ -1,7 +1,7 @@
 // hq_sweep.cu -- k_sweep, the persistent kernel of one directional update sweep
 // (src/dqmc_core.cpp:167-284) of every chain of a context: ONE launch per sweep.
 //
-// The grid holds one CTA of 8 warps per SM. Each CTA repeatedly takes a work item, the next
+// The grid holds one CTA of 8 warps per SM, as many as there are chains at most. Each CTA repeatedly takes a work item, the next
 // stabilisation interval of one chain, and runs all of it in the order of the launch sequence
 // it replaces:
 //   interval_body (wrap + Metropolis of the interval's slices, G resident in shared memory)
@@ -249,7 +249,9 @@ cudaError_t launch_sweep(const HqChain* chains, int nchains, const int2* cinfo, 
   cudaError_t e = cudaMemsetAsync(ctl, 0, sweep_ctl_ints(nchains) * sizeof(int), st);
   if (e != cudaSuccess) return e;
   if (nitems <= 0) return cudaSuccess;
-  k_sweep<<<std::min(grid, nitems), HQ_INT_THREADS, smem_sweep_bytes(Nmax, kmax), st>>>(
+  // A chain's intervals follow one another, so at most one item per chain is at work: a CTA beyond the
+  // chains would only wait, on an SM that other contexts could use.
+  k_sweep<<<std::min({grid, nitems, nchains}), HQ_INT_THREADS, smem_sweep_bytes(Nmax, kmax), st>>>(
       chains, nchains, cinfo, nitems, lists, nstab_max, dir, flags, ctl, clk);
   return cudaGetLastError();
 }

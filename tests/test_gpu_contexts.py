@@ -38,3 +38,22 @@ def test_a_context_of_smaller_chains_beside_a_larger_one(hq, mode):
         assert np.array_equal(x, y)
     for e in (a, b, c):
         e.close()
+
+
+@pytest.mark.parametrize("chains", [1, 3])
+def test_few_chains_hold_few_sms(hq, chains):
+    """A persistent sweep holds no more SMs than it has chains, the most that can be at work at once: a
+    CTA beyond them would only wait (its waits are counted when it takes an item), on an SM that other
+    contexts could use. An item's look at the queue takes a few thousand cycles, an interval of ten
+    8x8 slices some 400 thousand."""
+    e = hq.Engine([dict(nl=8, u=4.0, mu=0.1, beta=20.0, nt=200, stabilization_pace=10, seed=c) for c in range(chains)])
+    e.set_sweep_mode(hq.SWEEP_PERSISTENT)
+    e.fields_random()
+    e.init()
+    e.sweep(UP)
+    e.phase_cycles(reset=True)
+    e.sweep(DOWN, hq.capi.SWEEP_PHASE_CLOCKS)
+    pc = e.phase_cycles()
+    assert pc["items"] == 20 * chains
+    assert pc["wait"] < 0.25 * pc["interval"], pc
+    e.close()
