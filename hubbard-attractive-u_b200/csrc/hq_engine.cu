@@ -990,11 +990,12 @@ int hq_create(int device, int n_chains, const hq_chain_params* params, hq_ctx** 
     setup_sweep(c.get());
     // Small chains run persistently unless told otherwise: an interval takes them less time than the
     // launches and the gaps between them. One round trip of 40 slices, launches / persistent, ms: 64
-    // chains of 4x4 1.36 / 0.99, 6x6 2.59 / 2.14, 8x8 3.27 / 3.03, 9x9 5.20 / 5.66, 12x12 10.8 / 12.1;
-    // 256 chains of 6x6 4.19 / 4.15, 8x8 5.51 / 5.74. Larger chains gain more from the launch
-    // sequence's 16-warp factorisations and products over several SMs, and so do those of 7x7 and
-    // 8x8 once there are more of them than SMs.
-    if (c->sweep_capable && (c->Nmax <= 36 || (c->Nmax <= 64 && c->n <= c->sweep_grid)))
+    // chains of 4x4 1.39 / 1.01, 6x6 2.65 / 2.19, 8x8 3.37 / 3.09, 9x9 5.20 / 5.66, 12x12 10.8 / 12.1.
+    // Larger chains gain more from the launch sequence's 16-warp factorisations and products over
+    // several SMs, and so does any size once its chains have filled the SMs (one CTA each): 256 chains
+    // of 3x3 2.68 / 2.44, 4x4 1.99 / 1.88, 5x5 3.41 / 3.33, 6x6 4.25 / 4.15, 8x8 5.51 / 5.74; 296 of 4x4
+    // 2.08 / 2.12, 6x6 4.59 / 4.64; 1024 of 4x4 5.96 / 8.42, 6x6 14.9 / 17.5.
+    if (c->sweep_capable && ((c->Nmax <= 36 && 4 * c->n <= 7 * c->sweep_grid) || (c->Nmax <= 64 && c->n <= c->sweep_grid)))
       c->sweep_mode = HQ_SWEEP_PERSISTENT;
     // HQ_SWEEP_MODE=persistent | launches overrides the default mode (for comparisons)
     const char* m = std::getenv("HQ_SWEEP_MODE");

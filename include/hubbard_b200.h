@@ -188,8 +188,9 @@ HQ_API int hq_get_config(hq_ctx* ctx, int chain, int* expk_mode, int* delay_dept
  * Both give the same G and field trajectories. PERSISTENT needs every chain's matrices to fit
  * in one SM's shared memory (N <= 144 on B200); hq_set_sweep_mode returns HQ_E_RANGE
  * otherwise. Setting a mode drops the captured sweep graphs. hq_autotune picks the faster;
- * unless told otherwise a context runs PERSISTENT when every chain has at most 36 sites, or at
- * most 64 while there are no more chains than SMs, and LAUNCHES beyond that. */
+ * unless told otherwise a context runs PERSISTENT when every chain has at most 36 sites and there
+ * are no more than 7/4 chains per SM (259 on B200), or at most 64 sites and no more chains than
+ * SMs, and LAUNCHES beyond that. */
 #define HQ_SWEEP_LAUNCHES 0
 #define HQ_SWEEP_PERSISTENT 1
 HQ_API int hq_set_sweep_mode(hq_ctx* ctx, int mode);

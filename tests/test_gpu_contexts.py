@@ -57,3 +57,15 @@ def test_few_chains_hold_few_sms(hq, chains):
     assert pc["items"] == 20 * chains
     assert pc["wait"] < 0.25 * pc["interval"], pc
     e.close()
+
+
+@pytest.mark.parametrize("L,per_sm,persistent", [(1, 1.75, True), (1, 1.76, False), (6, 1.75, True), (6, 1.76, False),
+                                                 (4, 8.0, False)])
+def test_default_mode_of_many_small_chains(hq, L, per_sm, persistent, monkeypatch):
+    """Chains that outnumber the SMs by more than 7/4 gain from the launch sequence at any size."""
+    import torch
+    monkeypatch.delenv("HQ_SWEEP_MODE", raising=False)
+    n = int(per_sm * torch.cuda.get_device_properties(0).multi_processor_count + 0.5)
+    e = hq.Engine([dict(nl=L, u=4.0, mu=0.1, beta=0.2, nt=2, stabilization_pace=2, seed=c) for c in range(n)])
+    assert e.sweep_mode() == (hq.SWEEP_PERSISTENT if persistent else hq.SWEEP_LAUNCHES)
+    e.close()
