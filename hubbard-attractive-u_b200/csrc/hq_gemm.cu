@@ -158,14 +158,14 @@ __device__ __forceinline__ void gemm_tile(const HqGemmJob& J, int m0, int n0, do
 // interval has four instead of five of these launches and a dynamic one five instead of eight.
 template <int T>
 __global__ void __launch_bounds__(kGThreads<T>, GemmTile<T>::CTAS)
-k_gemm(HqGemmLists lists, int njobs, int tiles_n) {
+k_gemm(HqGemmLists lists, int tiles_n) {
   __shared__ __align__(16) double sA[2 * kGStage<T>];
   __shared__ __align__(16) double sB[2 * kGStage<T>];
   __shared__ double sK[2 * kGKc];
   __shared__ double red[32];
   __shared__ HqGemmJob J;
   static_assert(sizeof(HqGemmJob) == 128, "16 words of 8 bytes");
-  const int li = blockIdx.y / njobs, jb = blockIdx.y - li * njobs;
+  const int li = blockIdx.z, jb = blockIdx.y;
   if (threadIdx.x < 16) {
     const HqGemmJob* src = (li == 0 ? lists.l[0] : (li == 1 ? lists.l[1] : lists.l[2])) + jb;
     reinterpret_cast<unsigned long long*>(&J)[threadIdx.x] = reinterpret_cast<const unsigned long long*>(src)[threadIdx.x];
@@ -195,9 +195,9 @@ cudaError_t launch_gemm(const HqGemmLists& lists, int nlists, int njobs, int Mma
   auto padded = [&](int t) { return ((Mmax + t - 1) / t) * t * (((Nmax + t - 1) / t) * t); };
   const int t = padded(64) < padded(48) ? 64 : 48;
   const int tm = (Mmax + t - 1) / t, tn = (Nmax + t - 1) / t;
-  const dim3 grid(tm * tn, njobs * nlists);
-  if (t == 64) k_gemm<64><<<grid, kGThreads<64>, 0, st>>>(lists, njobs, tn);
-  else k_gemm<48><<<grid, kGThreads<48>, 0, st>>>(lists, njobs, tn);
+  const dim3 grid(tm * tn, njobs, nlists);  // up to 65535 jobs per list
+  if (t == 64) k_gemm<64><<<grid, kGThreads<64>, 0, st>>>(lists, tn);
+  else k_gemm<48><<<grid, kGThreads<48>, 0, st>>>(lists, tn);
   return cudaGetLastError();
 }
 cudaError_t launch_gemm(const HqGemmJob* jobs, int njobs, int Mmax, int Nmax, cudaStream_t st) {

@@ -69,3 +69,42 @@ def test_default_mode_of_many_small_chains(hq, L, per_sm, persistent, monkeypatc
     e = hq.Engine([dict(nl=L, u=4.0, mu=0.1, beta=0.2, nt=2, stabilization_pace=2, seed=c) for c in range(n)])
     assert e.sweep_mode() == (hq.SWEEP_PERSISTENT if persistent else hq.SWEEP_LAUNCHES)
     e.close()
+
+
+def _many(hq, n, **kw):
+    """n chains of 2 x 2, the last one with the parameters of the first and a seed of its own."""
+    cfg = [dict(nl=2, u=4.0, mu=0.1, beta=0.3, nt=3, stabilization_pace=2, seed=1 + (c % 7), **kw) for c in range(n)]
+    e, one = hq.Engine(cfg), hq.Engine([cfg[0], cfg[n - 1]])
+    for x in (e, one):
+        x.set_sweep_mode(hq.SWEEP_LAUNCHES)
+        x.fields_random()
+        x.init()
+    return e, one
+
+
+def test_displaced_sweep_of_22000_chains(hq):
+    """Three job lists of the displaced builder in one launch: more than 65535 products."""
+    n = 22000
+    e, one = _many(hq, n, dynamic=1)
+    for x in (e, one):
+        x.sweep(DYN, hq.SWEEP_MEASURE)
+        x.sweep(DOWN, hq.SWEEP_MEASURE)
+    for k, c in ((0, 0), (1, n - 1)):
+        assert np.array_equal(e.g(c), one.g(k))
+        assert np.array_equal(e.fields(c), one.fields(k))
+        for a, b in zip(e.dynamic_estimators(c), one.dynamic_estimators(k)):
+            assert np.array_equal(a, b)
+    e.close()
+    one.close()
+
+
+def test_adjoint_of_33000_chains(hq):
+    """The push with the first builder product in one launch: more than 65535 products."""
+    n = 33000
+    e, one = _many(hq, n)
+    (ld, gr), (ld1, gr1) = e.logdet_adjoint(), one.logdet_adjoint()
+    for k, c in ((0, 0), (1, n - 1)):
+        assert ld[c] == ld1[k] and gr[c][0] == gr1[k][0] and gr[c][1] == gr1[k][1]
+        assert np.array_equal(gr[c][2], gr1[k][2])
+    e.close()
+    one.close()
