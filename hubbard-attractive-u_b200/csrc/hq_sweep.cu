@@ -1,9 +1,9 @@
 // hq_sweep.cu -- k_sweep, the persistent kernel of one directional update sweep
 // (src/dqmc_core.cpp:167-284) of every chain of a context: ONE launch per sweep.
 //
-// The grid holds one CTA of 8 warps per SM, as many as there are chains at most. Each CTA repeatedly takes a work item, the next
-// stabilisation interval of one chain, and runs all of it in the order of the launch sequence
-// it replaces:
+// The grid holds one CTA of 8 warps per SM, as many as there are chains at most. Each CTA repeatedly
+// takes a work item, the next stabilisation interval of one chain, and runs all of it in the order of
+// the launch sequence it replaces:
 //   interval_body (wrap + Metropolis of the interval's slices, G resident in shared memory)
 //   bchain_body   (B products of the interval applied to the top of the pushing stack)
 //   udt_body      (UDV factorisation of the push)
