@@ -428,7 +428,8 @@ void build_jobs(hq_ctx* c) {
 // The finish of the log-det adjoint: Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T with Q the eigenbasis of
 // K. Q and the eigenvalues are constants of the chains' hopping matrices (one copy per distinct
 // lattice and parameters, one per custom matrix); the five products are batched jobs over all chains.
-void build_adjoint(hq_ctx* c) {
+// false: the device has no room for them (adjoint_on_host then takes their place).
+bool build_adjoint(hq_ctx* c) {
   size_t total = 0;
   auto take = [&](size_t bytes) { const size_t o = total; total += align256(bytes); return o; };
   std::map<std::tuple<int, double, double>, std::pair<size_t, size_t>> uniform;  // Q, w
@@ -459,7 +460,7 @@ void build_adjoint(hq_ctx* c) {
   char* base = nullptr;
   if (cudaMalloc(&base, total) != cudaSuccess) {
     cudaGetLastError();
-    throw HqError(HQ_E_NOMEM, "hq_logdet_adjoint: no room for " + std::to_string(total) + " bytes");
+    return false;
   }
   try {
     std::vector<double> w, Q;
@@ -504,6 +505,48 @@ void build_adjoint(hq_ctx* c) {
   c->d_adj_out = reinterpret_cast<double*>(base + o_out);
   c->d_adj_logdet = reinterpret_cast<double*>(base + o_ld);
   for (int k = 0; k < 5; ++k) c->adj_jobs[k] = reinterpret_cast<HqGemmJob*>(base + o_jobs[k]);
+  return true;
+}
+
+// The same finish without any device memory, for a context that all but fills the device: D and E^-1 are
+// read back chain by chain and multiplied here (a call for 64 chains of 100 sites, 60 slices: 210 ms
+// instead of 5.6).
+void adjoint_on_host(hq_ctx* c, double* out) {
+  std::map<std::tuple<int, double, double>, std::pair<std::vector<double>, std::vector<double>>> uniform;  // w, Q
+  HQ_CUDA(cudaStreamSynchronize(c->stream));
+  for (int i = 0; i < c->n; ++i) {
+    const ChainHost& h = c->ch[i];
+    const HqChain& d = c->desc[i];
+    const int N = h.N;
+    const size_t NN = size_t(N) * N;
+    if (!h.custom_hop) {
+      auto& u = uniform[std::make_tuple(h.p.nl, h.p.nnt, h.p.mu)];
+      if (u.first.empty()) {
+        u.first.resize(N);
+        u.second.resize(NN);
+        lattice_eig(h.p.nl, h.p.nnt, h.p.mu, u.first.data(), u.second.data());
+      }
+    }
+    const auto* u = h.custom_hop ? nullptr : &uniform[std::make_tuple(h.p.nl, h.p.nnt, h.p.mu)];
+    const std::vector<double>&w = u ? u->first : h.eig_w, &Q = u ? u->second : h.eig_Q;
+    std::vector<double> A(NN), B(NN), C(NN);
+    HQ_CUDA(cudaMemcpy(A.data(), d.inv_expK, NN * sizeof(double), cudaMemcpyDeviceToHost));
+    HQ_CUDA(cudaMemcpy(B.data(), d.W4, NN * sizeof(double), cudaMemcpyDeviceToHost));
+    host_gemm(N, A.data(), false, B.data(), false, C.data());  // E^-1 D
+    host_gemm(N, Q.data(), true, C.data(), false, A.data());   // Q^T E^-1 D
+    host_gemm(N, A.data(), false, Q.data(), false, B.data());  // Q^T E^-1 D Q
+    for (int j = 0; j < N; ++j)
+      for (int k = 0; k < N; ++k) {
+        const double dw = w[k] - w[j], fj = std::exp(-h.dt * w[j]);
+        const double phi = std::fabs(dw) > 1e-10 ? fj * std::expm1(-h.dt * dw) / dw : -h.dt * 0.5 * (std::exp(-h.dt * w[k]) + fj);
+        A[k + size_t(j) * N] = phi * B[j + size_t(k) * N];
+      }
+    host_gemm(N, Q.data(), false, A.data(), false, C.data());  // Q (Phi o (.)^T)
+    HQ_CUDA(cudaMemcpy(out, d.acc + HQ_ACC_DMU, sizeof(double), cudaMemcpyDeviceToHost));
+    HQ_CUDA(cudaMemcpy(out + 1, d.acc + HQ_ACC_DALPHA, sizeof(double), cudaMemcpyDeviceToHost));
+    host_gemm(N, C.data(), false, Q.data(), true, out + 2);    // Gamma
+    out += 2 + NN;
+  }
 }
 
 // The persistent sweep's scheduling data: per chain {n_stab, estimated cycles of one interval}
@@ -1638,7 +1681,7 @@ int hq_logdet_adjoint(hq_ctx* c, double* out, double* logdet) {
   if (!c || !out) throw HqError(HQ_E_INVALID, "null argument");
   if (!c->initialised || !c->at_zero) throw HqError(HQ_E_INVALID, "hq_logdet_adjoint: stacks must be at tau = 0");
   c->prof_next = 0;
-  if (!c->d_adj) build_adjoint(c);
+  const bool on_device = c->d_adj || build_adjoint(c);
   { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_adj_begin(c->d_desc, c->n, c->stream)); }
   // no-update up pass: wrap slice by slice, rebuild G from the stacks every pace slices
   // (the checkpoints), accumulate the adjoint contractions of every slice
@@ -1651,16 +1694,21 @@ int hq_logdet_adjoint(hq_ctx* c, double* out, double* logdet) {
   // log|det(1 + U D Vt)| = sum log dmax + log|det(dmax^-1 U^T + dmin Vt)| from the full left stack
   run_jobs(c, {PH_LOGDET}, 0, 0);
   run_jobs(c, {PH_LOGDET}, 0, 1);
-  { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_logdet(c->d_desc, c->n, c->d_adj_logdet, c->Nmax, c->resident, c->stream)); }
-  // Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T, Phi = divided differences of exp(-dt lambda)
-  for (int k = 0; k < 5; ++k) {
-    { ProfScope ps(c, PC_GEMM); HQ_CUDA(hq::launch_gemm(c->adj_jobs[k], c->n, c->Nmax, c->Nmax, c->stream)); }
-    if (k == 2) HQ_CUDA(hq::launch_adj_divided(c->d_desc, c->n, c->d_eig, c->stream));
-  }
-  HQ_CUDA(hq::launch_adj_gather(c->d_desc, c->n, c->d_adj_off, c->d_adj_out, c->stream));
-  HQ_CUDA(cudaMemcpyAsync(out, c->d_adj_out, c->adj_doubles * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  double* d_logdet = on_device ? c->d_adj_logdet : c->d_acc_all;  // (the gather buffer of the estimators has room for it)
+  { ProfScope ps(c, PC_ADJ); HQ_CUDA(hq::launch_logdet(c->d_desc, c->n, d_logdet, c->Nmax, c->resident, c->stream)); }
   if (logdet)
-    HQ_CUDA(cudaMemcpyAsync(logdet, c->d_adj_logdet, c->n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    HQ_CUDA(cudaMemcpyAsync(logdet, d_logdet, c->n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  if (on_device) {
+    // Gamma = Q (Phi o (Q^T E^-1 D Q)^T) Q^T, Phi = divided differences of exp(-dt lambda)
+    for (int k = 0; k < 5; ++k) {
+      { ProfScope ps(c, PC_GEMM); HQ_CUDA(hq::launch_gemm(c->adj_jobs[k], c->n, c->Nmax, c->Nmax, c->stream)); }
+      if (k == 2) HQ_CUDA(hq::launch_adj_divided(c->d_desc, c->n, c->d_eig, c->stream));
+    }
+    HQ_CUDA(hq::launch_adj_gather(c->d_desc, c->n, c->d_adj_off, c->d_adj_out, c->stream));
+    HQ_CUDA(cudaMemcpyAsync(out, c->d_adj_out, c->adj_doubles * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  } else {
+    adjoint_on_host(c, out);
+  }
   HQ_CUDA(cudaStreamSynchronize(c->stream));
   // the pass left the stacks at tau = beta
   c->at_zero = false;

@@ -151,6 +151,9 @@ HQ_API int hq_ratio_log(hq_ctx* ctx, int chain, long long capacity, double* out,
  * mu, alpha and the hopping matrix entries (dK_ij for K = -hop - mu): out per chain is
  * [dmu, dalpha, dK (N*N column-major)] and logdet[chain]. Runs a no-update pass with
  * stabilisation every `pace` slices; state must be at tau = 0 (after init or an up+down pair).
+ * The first call (and the first after hq_set_hopping) allocates device memory that the context
+ * keeps: the results, 2 + N*N doubles per chain, and an eigenbasis per distinct lattice and per
+ * custom hopping. Where the device has no room for it, the last step runs on the host instead.
  * No counterpart in the reference (new: adjoint of the log-determinant). */
 HQ_API int hq_logdet_adjoint(hq_ctx* ctx, double* out, double* logdet);
 
