@@ -18,10 +18,7 @@ constexpr int kCtaKc = 16, kCtaMaxB = 7;
 // Matrices of up to 64 rows, columns and K are staged whole: one fill, one barrier and then all of K,
 // instead of four chunks with a fill latency and two barriers each (64^3: 17.1k -> 13.4k cycles, 16^3: 5.7k -> 3.4k).
 constexpr int kCtaWhole = 64;
-#ifndef HQ_CTA_KK_UNROLL
-#define HQ_CTA_KK_UNROLL 4
-#endif
-constexpr int kCtaKkUnroll = HQ_CTA_KK_UNROLL;
+constexpr int kCtaKkUnroll = 4;
 
 __host__ __device__ constexpr inline int cta_pad16(int x) { return (x + 15) & ~15; }
 __host__ __device__ constexpr inline int cta_pad24(int x) { return ((x + 23) / 24) * 24; }
@@ -91,19 +88,10 @@ __device__ __forceinline__ void cta_stage8(const double* X, int ldx, bool kmaj, 
 }
 
 // C of job `job` for one transpose case (AMAJ: op(A) = A^T, contiguous along k; BMAJ: op(B) = B,
-// contiguous along k; KS: k-scalings). Inlined by default (HQ_CTA_NOINLINE=1 makes it a call):
-// measured 5-15% faster per product. `smem` holds cta_gemm_doubles(M, Nc) doubles, red >= 32
-// doubles. Every thread calls it.
-#ifndef HQ_CTA_NOINLINE
-#define HQ_CTA_NOINLINE 0
-#endif
-#if HQ_CTA_NOINLINE
-#define HQ_CTA_FN_ATTR __noinline__
-#else
-#define HQ_CTA_FN_ATTR __forceinline__
-#endif
+// contiguous along k; KS: k-scalings). Inlined: 5-15% faster per product than a call. `smem` holds
+// cta_gemm_doubles(M, Nc) doubles, red >= 32 doubles. Every thread calls it.
 template <bool AMAJ, bool BMAJ, bool KS, bool WHOLE>
-__device__ HQ_CTA_FN_ATTR void gemm_cta_t(const HqGemmJob& job, double* smem, double* red) {
+__device__ __forceinline__ void gemm_cta_t(const HqGemmJob& job, double* smem, double* red) {
   constexpr int kCtaKc = WHOLE ? kCtaWhole : hq::kCtaKc, kCtaStages = WHOLE ? 1 : hq::kCtaStages;
   constexpr int kCtaLdk = cta_ldk(kCtaKc);
   constexpr int kMaxB = WHOLE ? 2 : kCtaMaxB;  // 64 x 64: 12 blocks over 8 warps

@@ -38,8 +38,8 @@ template <int L>
 __device__ __noinline__ int metropolis_slice(const HqChain& ch, uint32_t rng, int flags, long long log_base) {
   extern __shared__ __align__(16) double smem[];
   // Warp 0 walks the next block beside the flush where the flush is long enough to lose a warp: round
-  // trips with / without, ms: 48 chains of 9 x 9 6.48 / 6.67, one of 8 x 8 10.07 / 10.06, 32 of 7 x 7
-  // 5.26 / 5.06. With G in global memory the flush is so long that the warp it lacks costs more than
+  // trips with / without, ms: 48 chains of 9 x 9 6.33 / 6.53, one of 8 x 8 13.6 / 13.2, 32 of 7 x 7 (dense)
+  // 5.67 / 5.46. With G in global memory the flush is so long that the warp it lacks costs more than
   // the walk beside it saves (16 chains of 14 x 14, interval kernel: 17.9 / 16.7 ms a sweep).
   constexpr bool kAhead = L >= 9;
   const int N = L > 0 ? L * L : ch.N;

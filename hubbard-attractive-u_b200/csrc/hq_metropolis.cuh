@@ -30,12 +30,12 @@ namespace hq {
 //  On lattices of 81 sites and more with G in shared memory, warps 1 .. 7 flush while warp 0 takes the
 //  next block's g = G[B', B'] + X[B', :] Y[:, B'] (the same DMMA steps, so the same bits as the flush
 //  leaves) and walks it.
-//  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 40, 18, 46 one
+//  Measured at 12 x 12, 8 warps, thousands of cycles per slice (walk, panels, flush): 42, 17, 46 one
 //  after the other; 56, 28 and 85 with predicated record stores in the walk, a branch per flip in the
 //  panels, and a flush that checked every element against the edge.
 //  The walk and the panels are bound by the latency of one dependency chain, the flush by the DMMA
 //  pipe. With the walks beside the flushes a round trip of 200 slices at 12 x 12 takes 256 chains
-//  56.3 ms instead of 60.5, one chain 23.0 instead of 25.5.
+//  48.2 ms instead of 51.1 (launches), one chain 23.6 instead of 25.3.
 // ---------------------------------------------------------------------------------
 constexpr int kLdR = 18;  // leading dimension of the walk's records: 16-byte rows whose stores spread over the banks
 
@@ -158,19 +158,20 @@ __device__ __forceinline__ bool walk_block16(const double* g, int ld, const Metr
   return false;
 }
 
-// the walks of the ratio log, of near ties and of short blocks, out of line: their code and
-// registers do not weigh on the fast walk's
+// The walks of the ratio log, of near ties and of short blocks, out of line behind one call each: their
+// code and registers do not weigh on the fast walk's (a call of its own per length cost 1 % at 8x8). Blocks
+// of 4 and 8 sites (the smaller delay depths, last blocks such as those of 36 and 100 sites) and single
+// last sites (49, 81, 225 sites) have their steps and loads fixed at compile time. Round trips of 40
+// slices, launches, nb at run time / fixed, ms: 64 chains of 8x8 at depth 4 5.59 / 3.99, at 8 4.46 / 3.73; 128
+// of 12x12 16.3 / 13.7, 13.3 / 11.9; 16 of 14x14 76.6 / 71.4, 55.2 / 52.8; 64 of 6x6 at depth 16 2.70 / 2.53.
 template <bool EXACT, bool LOGT>
 __device__ __noinline__ bool walk_rare(const double* g, int ld, const MetroShared sh, int b0, int nb, int slot) {
+  if constexpr (!EXACT && !LOGT) {
+    if (nb == 1) return walk_block16<EXACT, LOGT, 1>(g, ld, sh, b0, nb, slot);
+    if (nb == 4) return walk_block16<EXACT, LOGT, 4>(g, ld, sh, b0, nb, slot);
+    if (nb == 8) return walk_block16<EXACT, LOGT, 8>(g, ld, sh, b0, nb, slot);
+  }
   return walk_block16<EXACT, LOGT, 0>(g, ld, sh, b0, nb, slot);
-}
-// The walks of blocks of 4 and 8 sites (the smaller delay depths, last blocks such as those of 36 and 100
-// sites), their steps and loads fixed at compile time. Round trips of 40 slices, launches, nb at run time /
-// fixed, ms: 64 chains of 8x8 at depth 4 5.59 / 4.03, at 8 4.47 / 3.69; 128 of 12x12 16.3 / 13.7, 13.3 / 11.7; 16
-// of 14x14 76.7 / 71.7, 55.1 / 53.1; 64 of 6x6 at depth 16 2.70 / 2.52.
-template <int NBC>
-__device__ __noinline__ bool walk_depth(const double* g, int ld, const MetroShared sh, int b0, int slot) {
-  return walk_block16<false, false, NBC>(g, ld, sh, b0, NBC, slot);
 }
 // the walk with the reference's form of every decision where the fast one came near a tie; again()
 // restores g before a second walk, if the first one's records overwrote it
@@ -181,10 +182,7 @@ __device__ __forceinline__ void walk(const double* g, int ld, const MetroShared&
   } else if (nb == 16) {
     if (walk_block16<false, false, 16>(g, ld, sh, b0, nb, slot)) again(), walk_rare<true, false>(g, ld, sh, b0, nb, slot);
   } else {
-    const bool near = nb == 8   ? walk_depth<8>(g, ld, sh, b0, slot)
-                      : nb == 4 ? walk_depth<4>(g, ld, sh, b0, slot)
-                                : walk_rare<false, false>(g, ld, sh, b0, nb, slot);
-    if (near) again(), walk_rare<true, false>(g, ld, sh, b0, nb, slot);
+    if (walk_rare<false, false>(g, ld, sh, b0, nb, slot)) again(), walk_rare<true, false>(g, ld, sh, b0, nb, slot);
   }
 }
 // the walk of a tile that lies in G
