@@ -380,10 +380,10 @@ def run_gpu(args):
     traffic = None
     if dom_name == "interval" and metric_wl:
         # DRAM bytes of one k_interval launch: ncu capture of a 16-chain launch of this workload
-        # (2.864 MB read, 0 written: the chains' G and fields), scaled by the chains of one launch
+        # (2.91 MB read and written: the chains' G and fields), scaled by the chains of one launch
         # here (the traffic is per-chain state; with two chain groups a launch covers half of them)
         chains_per_launch = n * (CFG["nt"] // CFG["stabilization_pace"]) * args.steps / max(1, int(cnt_cls[dom]))
-        traffic = 2.864e6 * chains_per_launch / 16
+        traffic = 2.91e6 * chains_per_launch / 16
     f_sweep = world * sum(dense_equivalent_flops(p, args.steps, acc_chain[c]) for c, p in enumerate(params))
     sweep_tf = f_sweep / (ms * 1e-3) / 1e12
     sweep_mode = "persistent" if eng.sweep_mode() == hq.SWEEP_PERSISTENT else "launches"
