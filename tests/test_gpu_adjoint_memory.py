@@ -6,6 +6,8 @@ orthogonal or, like Phi, smaller than one. FP64 sums on the device against exten
 differ by less than 5 N 2^-53 sqrt(N) max|E^-1 D| < 1e-11 times the largest gradient (the entries of dK
 are of order one, |E^-1 D| of order nt / dK's dt nt = 10 times as large). The log-determinant, mu's and
 alpha's gradients come from the same kernels: the same bits."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -34,6 +36,7 @@ def test_adjoint_without_room_on_the_device(hq, bonds):
     ld, grads = a.logdet_adjoint()  # also loads every kernel before the device is filled
     a.close()
     b = make()
+    gc.collect()  # no context of an earlier test gives its memory back later
     # the results alone take 5 MB; leave the device 2 to 4 MB
     blocks = []
     for room in (64 << 20, 4 << 20):
